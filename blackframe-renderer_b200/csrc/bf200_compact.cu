@@ -27,22 +27,25 @@ __device__ __forceinline__ uint32_t key_at(const uint8_t* keys, uint32_t n, uint
     return slot < n ? static_cast<uint32_t>(keys[slot]) : 0xFFU;
 }
 
+// MAX: compiled route limit (4 for the shadow queue, the sort and the public call, kCompactMaxRoutes
+// for shading), so that few routes do not pay for the ballots of many.
+template <uint32_t MAX>
 __global__ void __launch_bounds__(256) k_compact_count(const uint8_t* __restrict__ keys, uint32_t n, uint32_t routes,
                                                        uint32_t tiles, uint32_t* __restrict__ tile_counts) {
-    __shared__ uint32_t partial[kCompactWarps][kCompactMaxRoutes];
+    __shared__ uint32_t partial[kCompactWarps][MAX];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31U;
     const uint32_t first = blockIdx.x * kCompactTile + warp * kWarpSlots;
-    uint32_t count[kCompactMaxRoutes] = {0U, 0U, 0U, 0U};
+    uint32_t count[MAX] = {};
     for (uint32_t step = 0; step < kWarpSlots; step += 32U) {
         const uint32_t key = key_at(keys, n, first + step + lane);
 #pragma unroll
-        for (uint32_t r = 0; r < kCompactMaxRoutes; ++r) {
+        for (uint32_t r = 0; r < MAX; ++r) {
             count[r] += __popc(__ballot_sync(0xFFFFFFFFU, key == r && r < routes));
         }
     }
     if (lane == 0U) {
 #pragma unroll
-        for (uint32_t r = 0; r < kCompactMaxRoutes; ++r) {
+        for (uint32_t r = 0; r < MAX; ++r) {
             partial[warp][r] = count[r];
         }
     }
@@ -92,24 +95,25 @@ __global__ void __launch_bounds__(kScanThreads) k_compact_scan(uint32_t* __restr
     }
 }
 
+template <uint32_t MAX>
 __global__ void __launch_bounds__(256) k_compact_scatter(const uint8_t* __restrict__ keys, uint32_t n,
                                                          uint32_t routes, uint32_t tiles,
                                                          const uint32_t* __restrict__ tile_offsets,
                                                          uint32_t* __restrict__ queue, uint8_t* __restrict__ reset_keys) {
-    __shared__ uint32_t warp_base[kCompactWarps][kCompactMaxRoutes];
+    __shared__ uint32_t warp_base[kCompactWarps][MAX];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31U;
     const uint32_t first = blockIdx.x * kCompactTile + warp * kWarpSlots;
-    uint32_t count[kCompactMaxRoutes] = {0U, 0U, 0U, 0U};
+    uint32_t count[MAX] = {};
     for (uint32_t step = 0; step < kWarpSlots; step += 32U) {
         const uint32_t key = key_at(keys, n, first + step + lane);
 #pragma unroll
-        for (uint32_t r = 0; r < kCompactMaxRoutes; ++r) {
+        for (uint32_t r = 0; r < MAX; ++r) {
             count[r] += __popc(__ballot_sync(0xFFFFFFFFU, key == r && r < routes));
         }
     }
     if (lane == 0U) {
 #pragma unroll
-        for (uint32_t r = 0; r < kCompactMaxRoutes; ++r) {
+        for (uint32_t r = 0; r < MAX; ++r) {
             warp_base[warp][r] = count[r];
         }
     }
@@ -124,9 +128,9 @@ __global__ void __launch_bounds__(256) k_compact_scatter(const uint8_t* __restri
         }
     }
     __syncthreads();
-    uint32_t base[kCompactMaxRoutes];
+    uint32_t base[MAX];
 #pragma unroll
-    for (uint32_t r = 0; r < kCompactMaxRoutes; ++r) {
+    for (uint32_t r = 0; r < MAX; ++r) {
         base[r] = r < routes ? warp_base[warp][r] : 0U;
     }
     const uint32_t below = (1U << lane) - 1U;
@@ -134,7 +138,7 @@ __global__ void __launch_bounds__(256) k_compact_scatter(const uint8_t* __restri
         const uint32_t slot = first + step + lane;
         const uint32_t key = key_at(keys, n, slot);
 #pragma unroll
-        for (uint32_t r = 0; r < kCompactMaxRoutes; ++r) {
+        for (uint32_t r = 0; r < MAX; ++r) {
             const bool mine = key == r && r < routes;
             const unsigned ballot = __ballot_sync(0xFFFFFFFFU, mine);
             if (mine) {
@@ -157,9 +161,19 @@ cudaError_t launch_compaction(const uint8_t* keys, uint32_t n, uint32_t routes, 
         return cudaErrorInvalidValue;
     }
     const uint32_t tiles = n == 0U ? 1U : (n + kCompactTile - 1U) / kCompactTile;
-    k_compact_count<<<tiles, 256, 0, stream>>>(keys, n, routes, tiles, tile_counts);
+    if (routes <= kCompactFewRoutes) {
+        k_compact_count<kCompactFewRoutes><<<tiles, 256, 0, stream>>>(keys, n, routes, tiles, tile_counts);
+    } else {
+        k_compact_count<kCompactMaxRoutes><<<tiles, 256, 0, stream>>>(keys, n, routes, tiles, tile_counts);
+    }
     k_compact_scan<<<1, kScanThreads, 0, stream>>>(tile_counts, routes, tiles, offsets, total);
-    k_compact_scatter<<<tiles, 256, 0, stream>>>(keys, n, routes, tiles, tile_counts, queue, reset_keys);
+    if (routes <= kCompactFewRoutes) {
+        k_compact_scatter<kCompactFewRoutes>
+            <<<tiles, 256, 0, stream>>>(keys, n, routes, tiles, tile_counts, queue, reset_keys);
+    } else {
+        k_compact_scatter<kCompactMaxRoutes>
+            <<<tiles, 256, 0, stream>>>(keys, n, routes, tiles, tile_counts, queue, reset_keys);
+    }
     *launches += 3U;
     return cudaGetLastError();
 }

@@ -122,14 +122,20 @@ struct TransportParams {
 };
 
 // Shading routes. A hit is shaded by the kernel specialised for its material's single closure
-// kind; misses and every other material take the generic kernel.
-constexpr uint32_t kRouteGeneric = 0U, kRouteLambert = 1U, kRouteConductor = 2U, kRouteDielectric = 3U;
-constexpr uint32_t kRouteCount = 4U;
+// kind; misses (route 0) and every other material (routes 1 to kGenericRoutes - 1, one per sequence
+// of closure kinds, the last for all further ones) take the generic kernel, which runs over its
+// routes one after another so that a warp's lanes share a sequence. With one generic route a warp's
+// lanes, and the warps of an SM, were at different closures' code all the time: on the layered Cornell
+// box (333 x 217 x 23) shading took 31.5 ms, now 8.9 ms (8 generic routes, shared code copies).
+constexpr uint32_t kGenericRoutes = 8U, kRouteMiss = 0U;
+constexpr uint32_t kRouteLambert = 8U, kRouteConductor = 9U, kRouteDielectric = 10U;
+constexpr uint32_t kRouteCount = 11U;
 constexpr uint8_t kRouteNone = 0xFFU;  // slot not shaded this iteration / no shadow ray
 
 // Stable compaction tiles: one 256-thread block per 4096 consecutive slots.
 constexpr uint32_t kCompactTile = 4096U;
-constexpr uint32_t kCompactMaxRoutes = 4U;
+constexpr uint32_t kCompactMaxRoutes = kRouteCount;
+constexpr uint32_t kCompactFewRoutes = 4U;
 
 // Slot states of the persistent wavefront.
 constexpr uint8_t kSlotEmpty = 0, kSlotActive = 1, kSlotDone = 2;

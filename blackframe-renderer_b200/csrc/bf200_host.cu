@@ -1100,7 +1100,7 @@ uint64_t film_samples_per_chunk(uint64_t pixels, uint64_t samples_per_pixel) {
 // The wavefront over no more slots than the trace has paths. Every stage and both compactions walk
 // all slots in each iteration, so a short trace pays for slots it never fills: with the default
 // 2,097,152 slots, 4,096 paths of the plain Cornell box took 2.15 ms (57 us an iteration in k_trace's
-// slot fetch alone), and 1.31 ms with 4,096 slots. Which slot a path runs in changes none of its results.
+// slot fetch alone), and 1.38 ms with 4,096 slots. Which slot a path runs in changes none of its results.
 Wavefront fit_slots(const Wavefront& w, uint64_t paths) {
     Wavefront fitted = w;
     fitted.capacity = static_cast<uint32_t>(std::min<uint64_t>(w.capacity, std::max<uint64_t>(1, paths)));
@@ -1756,18 +1756,29 @@ BF200_EXPORT blackframe_status bf200_scene_create(bf200_context* c, const bf200_
         }
         scene->plain_materials = plain_materials;
         // shading route of a hit on each instance: the kernel specialised for its material's single
-        // closure kind, or the generic one (several closures, or another kind)
-        std::vector<uint8_t> inst_route(d->instance_count, static_cast<uint8_t>(kRouteGeneric));
+        // closure kind, or the generic one (several closures, or another kind), whose routes are dealt
+        // to the sequences of closure kinds in the order the instances use them
+        std::vector<uint8_t> inst_route(d->instance_count);
+        std::vector<std::vector<uint32_t>> sequences;
         for (uint32_t i = 0; i < d->instance_count; ++i) {
-            const uint32_t m = d->instances[i].material_index;
-            if (d->materials[m].closure_count != 1) {
-                continue;
+            const auto& mat = d->materials[d->instances[i].material_index];
+            std::vector<uint32_t> kinds(mat.closure_count);
+            for (uint32_t k = 0; k < mat.closure_count; ++k) {
+                kinds[k] = d->closures[mat.closure_offset + k].kind;
             }
-            switch (closures[m].kind) {
-                case kClosureLambert: inst_route[i] = static_cast<uint8_t>(kRouteLambert); break;
-                case kClosureConductor: inst_route[i] = static_cast<uint8_t>(kRouteConductor); break;
-                case kClosureDielectric: inst_route[i] = static_cast<uint8_t>(kRouteDielectric); break;
-                default: break;
+            const uint32_t only = kinds.size() == 1 ? kinds[0] : 0U;
+            if (only == kClosureLambert) {
+                inst_route[i] = static_cast<uint8_t>(kRouteLambert);
+            } else if (only == kClosureConductor) {
+                inst_route[i] = static_cast<uint8_t>(kRouteConductor);
+            } else if (only == kClosureDielectric) {
+                inst_route[i] = static_cast<uint8_t>(kRouteDielectric);
+            } else {
+                size_t at = std::find(sequences.begin(), sequences.end(), kinds) - sequences.begin();
+                if (at == sequences.size() && at + 2U < kGenericRoutes) {
+                    sequences.push_back(kinds);
+                }
+                inst_route[i] = static_cast<uint8_t>(std::min<size_t>(1U + at, kGenericRoutes - 1U));
             }
         }
         stats.instance_ms = ms_since(t_instances);
@@ -3415,7 +3426,7 @@ BF200_EXPORT blackframe_status bf200_compact_routes_device(bf200_context* c, con
     if (c == nullptr || offsets == nullptr || (n != 0 && (keys == nullptr || queue == nullptr))) {
         return fail(c, BLACKFRAME_STATUS_INVALID_ARGUMENT, "null argument");
     }
-    if (routes == 0U || routes > kCompactMaxRoutes) {
+    if (routes == 0U || routes > kCompactFewRoutes) {
         return fail(c, BLACKFRAME_STATUS_OUT_OF_RANGE, "routes must be 1..4");
     }
     if (cudaSetDevice(c->device) != cudaSuccess) {

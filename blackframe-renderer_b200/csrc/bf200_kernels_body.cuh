@@ -1105,7 +1105,7 @@ __device__ __forceinline__ void trace_finish(const SceneView& s, const Wavefront
     }
     if (c.instance == 0xFFFFFFFFU) {
         w.hit_id[slot] = make_uint2(0xFFFFFFFFU, 0U);
-        w.route[slot] = static_cast<uint8_t>(kRouteGeneric);
+        w.route[slot] = static_cast<uint8_t>(kRouteMiss);
         return;
     }
     TriangleHit th;
@@ -2062,20 +2062,20 @@ __device__ __forceinline__ void adjoint_flush(double* sum, double* gradients) {
     }
 }
 
-// One launch per route: K is the closure kind the route's slots all share (0: generic route,
-// misses and any other material). The route queue lists the route's slots in slot order.
+// Shades the slots of routes [first_route, end_route). K is the closure kind they all share (0: the
+// generic routes, misses and any other material). The queue lists each route's slots in slot order.
 // ADJ: the replay of the path-replay adjoint (`a` is read only then).
 // K: closure kind (0 reads it from the record); ADJ: path-replay adjoint; CONE: the slots carry ray
 // cones (the cone column is read and written only then); TREE: lights are selected by the scene's
 // spatial light tree.
 template <int K, bool ADJ, bool CONE, bool TREE>
 __global__ void __launch_bounds__(256, BF200_SHADE_MIN_BLOCKS) k_shade(SceneView s, Wavefront w, PathSource src, TransportParams p,
-                                               uint32_t route, AdjointView a) {
+                                               uint32_t first_route, uint32_t end_route, AdjointView a) {
     __shared__ double adjoint_sum[ADJ ? kAdjointWords : 1];
     if constexpr (ADJ) {
         adjoint_zero(adjoint_sum);
     }
-    const uint32_t begin = w.route_offsets[route], end = w.route_offsets[route + 1U];
+    const uint32_t begin = w.route_offsets[first_route], end = w.route_offsets[end_route];
     const uint32_t stride = gridDim.x * blockDim.x;
     uint32_t active_here = 0;
     // the reference's stage counts, kept by the cone-carrying instantiations only: closure samples,
@@ -2728,32 +2728,45 @@ __global__ void __launch_bounds__(128) k_query_occlusion(SceneView s, const bf20
     }
 }
 
-// The four shading kernels of one wavefront iteration, one per route.
+// The shading kernels of one wavefront iteration: the Lambert route's, and the others.
 template <bool ADJ, bool CONE, bool TREE>
-void launch_shading(const SceneView& s, const Wavefront& w, const PathSource& src, const TransportParams& p,
-                    uint32_t grid, const AdjointView& a, cudaStream_t stream) {
-    k_shade<0, ADJ, CONE, TREE><<<grid, 256, 0, stream>>>(s, w, src, p, kRouteGeneric, a);
-    k_shade<static_cast<int>(kClosureLambert), ADJ, CONE, TREE><<<grid, 256, 0, stream>>>(s, w, src, p,
-                                                                                           kRouteLambert, a);
-    k_shade<static_cast<int>(kClosureConductor), ADJ, CONE, TREE><<<grid, 256, 0, stream>>>(s, w, src, p,
-                                                                                             kRouteConductor, a);
-    k_shade<static_cast<int>(kClosureDielectric), ADJ, CONE, TREE><<<grid, 256, 0, stream>>>(s, w, src, p,
-                                                                                              kRouteDielectric, a);
+void launch_shade_lambert(const SceneView& s, const Wavefront& w, const PathSource& src, const TransportParams& p,
+                          uint32_t grid, const AdjointView& a, cudaStream_t stream) {
+    k_shade<static_cast<int>(kClosureLambert), ADJ, CONE, TREE>
+        <<<grid, 256, 0, stream>>>(s, w, src, p, kRouteLambert, kRouteLambert + 1U, a);
+}
+
+template <bool ADJ, bool CONE, bool TREE>
+void launch_shade_others(const SceneView& s, const Wavefront& w, const PathSource& src, const TransportParams& p,
+                         uint32_t grid, const AdjointView& a, cudaStream_t stream) {
+    k_shade<0, ADJ, CONE, TREE><<<grid, 256, 0, stream>>>(s, w, src, p, 0U, kGenericRoutes, a);
+    k_shade<static_cast<int>(kClosureConductor), ADJ, CONE, TREE>
+        <<<grid, 256, 0, stream>>>(s, w, src, p, kRouteConductor, kRouteConductor + 1U, a);
+    k_shade<static_cast<int>(kClosureDielectric), ADJ, CONE, TREE>
+        <<<grid, 256, 0, stream>>>(s, w, src, p, kRouteDielectric, kRouteDielectric + 1U, a);
 }
 
 #ifdef BF200_KERNELS_MAIN_TU
 // The shading launchers are instantiated in their own translation units (bf200_shade_*.cu), which
 // compile in parallel.
-extern template void launch_shading<false, false, false>(const SceneView&, const Wavefront&, const PathSource&,
-    const TransportParams&, uint32_t, const AdjointView&, cudaStream_t);
-extern template void launch_shading<false, true, false>(const SceneView&, const Wavefront&, const PathSource&,
-    const TransportParams&, uint32_t, const AdjointView&, cudaStream_t);
-extern template void launch_shading<false, false, true>(const SceneView&, const Wavefront&, const PathSource&,
-    const TransportParams&, uint32_t, const AdjointView&, cudaStream_t);
-extern template void launch_shading<false, true, true>(const SceneView&, const Wavefront&, const PathSource&,
-    const TransportParams&, uint32_t, const AdjointView&, cudaStream_t);
-extern template void launch_shading<true, false, false>(const SceneView&, const Wavefront&, const PathSource&,
-    const TransportParams&, uint32_t, const AdjointView&, cudaStream_t);
+#define BF200_SHADE_LAUNCHERS(ADJ, CONE, TREE)                                                                    \
+    extern template void launch_shade_lambert<ADJ, CONE, TREE>(const SceneView&, const Wavefront&,               \
+        const PathSource&, const TransportParams&, uint32_t, const AdjointView&, cudaStream_t);                  \
+    extern template void launch_shade_others<ADJ, CONE, TREE>(const SceneView&, const Wavefront&,                \
+        const PathSource&, const TransportParams&, uint32_t, const AdjointView&, cudaStream_t);
+BF200_SHADE_LAUNCHERS(false, false, false)
+BF200_SHADE_LAUNCHERS(false, true, false)
+BF200_SHADE_LAUNCHERS(false, false, true)
+BF200_SHADE_LAUNCHERS(false, true, true)
+BF200_SHADE_LAUNCHERS(true, false, false)
+#undef BF200_SHADE_LAUNCHERS
+
+template <bool ADJ, bool CONE, bool TREE>
+void launch_shading(const SceneView& s, const Wavefront& w, const PathSource& src, const TransportParams& p,
+                    uint32_t grid, const AdjointView& a, cudaStream_t stream) {
+    launch_shade_lambert<ADJ, CONE, TREE>(s, w, src, p, grid, a, stream);
+    launch_shade_others<ADJ, CONE, TREE>(s, w, src, p, grid, a, stream);
+}
 
 // ------------------------------------------------------------------------------------------------
 // k_iteration_gate: the end of one wavefront iteration inside a graph's device-side loop

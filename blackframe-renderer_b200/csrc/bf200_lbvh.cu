@@ -316,7 +316,7 @@ cudaError_t build_blas_lbvh(const float* positions, uint32_t vertex_count, const
     //  9 sort order, 10 digits, 11 compaction tile counts, 12 centroid bounds and route offsets,
     //  13 BVH2 nodes, 14 parents + arrival counters + ranges, 15 leaf records
     const size_t sizes[16] = {bytes_positions, bytes_triangles, 16ULL * n, 16ULL * n, 16ULL * n, 8ULL * n, 8ULL * n,
-                              4ULL * n, 4ULL * n, 4ULL * n, static_cast<size_t>(n), 4ULL * kCompactMaxRoutes * tiles,
+                              4ULL * n, 4ULL * n, 4ULL * n, static_cast<size_t>(n), 4ULL * kCompactFewRoutes * tiles,
                               64, sizeof(BvhNode) * (n - 1), 8ULL * (n - 1) + 16 + 16ULL * (n - 1), 48ULL * n};
     size_t offsets[16] = {};
     size_t total = 0;
@@ -375,7 +375,7 @@ cudaError_t build_blas_lbvh(const float* positions, uint32_t vertex_count, const
         k_lbvh_digits<<<blocks(n), kLbvhThreads, 0, stream>>>(keys[cur], n, static_cast<uint32_t>(shift), digits);
         e = cudaGetLastError();
         if (e == cudaSuccess) {
-            e = launch_compaction(digits, n, kCompactMaxRoutes, tile_counts, order, small + 8, nullptr, nullptr,
+            e = launch_compaction(digits, n, kCompactFewRoutes, tile_counts, order, small + 8, nullptr, nullptr,
                                   stream, &launches);
         }
         if (e == cudaSuccess) {

@@ -2,6 +2,6 @@
 #include "bf200_kernels_body.cuh"
 
 namespace bf200 {
-template void launch_shading<true, false, false>(const SceneView&, const Wavefront&, const PathSource&,
-                                             const TransportParams&, uint32_t, const AdjointView&, cudaStream_t);
+template void launch_shade_others<true, false, false>(const SceneView&, const Wavefront&, const PathSource&, const TransportParams&,
+                                    uint32_t, const AdjointView&, cudaStream_t);
 }  // namespace bf200

@@ -10,6 +10,21 @@
 
 #include "bf200_geometry.cuh"
 
+// One out-of-line copy of a function that the shading kernels call from several places. With every
+// call inlined the kernels were 284 KB (Lambert) to 1 MB (generic) of code, far beyond the
+// instruction cache, and their warps waited for instructions (no_instruction stalls per issue:
+// 2.6 Lambert, 10 conductor, 8 dielectric, 65 generic).
+#define BF_SHARED static __device__ __noinline__
+// The same for the small vector and product blocks, except in the Lambert kernels (BF_SHADE_INLINE):
+// they call few of them, fit well enough, and lose more to the calls' register moves than they gain
+// (Cornell box with spheres, 256 spp: shading 45 ms with the Lambert kernel's blocks inlined, 53 ms
+// out of line; BVH-stress frame, 16 spp, where conductors and dielectrics weigh more: 50 and 44 ms).
+#ifdef BF_SHADE_INLINE
+#define BF_BLOCK __device__ __forceinline__
+#else
+#define BF_BLOCK BF_SHARED
+#endif
+
 namespace bf200 {
 
 constexpr float kInf = __builtin_huge_valf();
@@ -53,9 +68,9 @@ __device__ __forceinline__ float max_abs3(F3 v) {
 }
 __device__ __forceinline__ F3 ld3(const float4 v) { return {v.x, v.y, v.z}; }
 
-// Sine and cosine of a float angle: the double-precision values rounded once to float. One
-// out-of-line copy shared by every call site (one argument reduction for both values).
-static __device__ __noinline__ float2 sincos_f(float a) {
+// Sine and cosine of a float angle: the double-precision values rounded once to float (one argument
+// reduction for both values).
+BF_SHARED float2 sincos_f(float a) {
     double s = 0.0, c = 0.0;
     sincos(static_cast<double>(a), &s, &c);
     return make_float2(static_cast<float>(s), static_cast<float>(c));
@@ -144,6 +159,10 @@ struct Stream {
             const uint64_t bits = mix_bits(state ^ dimension);
             return static_cast<float>(bits >> 40U) * 0x1p-24F;
         }
+        return owen_sample(sobol, sample, seed, pixel_hash, dimension);
+    }
+    BF_SHARED float owen_sample(const uint32_t* sobol, uint64_t sample, uint64_t seed,
+                                                     uint64_t pixel_hash, uint64_t dimension) {
         const uint64_t sd = transport_sobol_dimension(dimension);
         const uint32_t* heads = sobol + 64ULL * sd;
         uint64_t gray = sample ^ (sample >> 1U);
@@ -164,7 +183,7 @@ __device__ __forceinline__ uint64_t bounce_base(uint32_t bounce) { return 4ULL +
 // Frames and directions (LocalFrame.hpp, BsdfOnlyPathLoop.hpp:190-209)
 // ------------------------------------------------------------------------------------------------
 
-__device__ __forceinline__ F3 robust_unit(F3 d, Lane& lane) {
+BF_BLOCK F3 robust_unit(F3 d, Lane& lane) {
     if (!finite3(d)) {
         lane.fail();
         return d;
@@ -200,7 +219,7 @@ struct Frame {
     }
 };
 
-__device__ __forceinline__ F3 robust_unit_vector(F3 v, Lane& lane) {
+BF_BLOCK F3 robust_unit_vector(F3 v, Lane& lane) {
     const float m = max_abs3(v);
     if (!finite3(v) || m == 0.0F) {
         lane.fail();
@@ -219,7 +238,7 @@ __device__ __forceinline__ bool orthonormal(F3 t, F3 b, F3 n) {
 }
 
 // LocalFrame.hpp:188-219
-__device__ __forceinline__ Frame frame_from_unit_normal_and_tangent(F3 n, F3 tangent, Lane& lane) {
+BF_BLOCK Frame frame_from_unit_normal_and_tangent(F3 n, F3 tangent, Lane& lane) {
     const F3 td = robust_unit_vector(tangent, lane);
     const F3 projected = td - n * dot(td, n);
     F3 ut = robust_unit_vector(projected, lane);
@@ -250,8 +269,8 @@ __device__ __forceinline__ Frame frame_from_normal(F3 v, Lane& lane) {
 
 // LocalFrame.hpp:116-135
 __device__ __forceinline__ Frame rotated_about_normal(const Frame& f, float angle, Lane& lane) {
-    const float reduced = remainderf(angle, 2.0F * kPi);
-    const float2 sc = sincos_f(reduced);
+    // an unrotated frame has sine `angle` (a zero of its sign) and cosine 1
+    const float2 sc = angle == 0.0F ? make_float2(angle, 1.0F) : sincos_f(remainderf(angle, 2.0F * kPi));
     const float c = sc.y;
     const float s = sc.x;
     const F3 rotated = f.t * c + f.b * s;
@@ -269,7 +288,7 @@ __device__ __forceinline__ float outward(float value, float off) {
     return value;
 }
 
-__device__ __forceinline__ F3 offset_ray_origin(F3 p, F3 err, F3 ng, F3 w, Lane& lane) {
+BF_BLOCK F3 offset_ray_origin(F3 p, F3 err, F3 ng, F3 w, Lane& lane) {
     const float m = max_abs3(ng);
     const F3 sn = ng / m;
     const F3 n = sn / sqrtf(dot(sn, sn));
@@ -312,7 +331,7 @@ __device__ __forceinline__ F3 offset_surface_point(F3 p, F3 err, F3 ng, F3 w, La
 }
 
 // ShadowRay.hpp:107-135
-__device__ __forceinline__ void unit_segment(F3 origin, F3 endpoint, F3 expected, F3& direction,
+BF_BLOCK void unit_segment(F3 origin, F3 endpoint, F3 expected, F3& direction,
                                              float& length, Lane& lane) {
     const F3 disp = endpoint - origin;
     const float scale = max_abs3(disp);
@@ -339,15 +358,30 @@ __device__ __forceinline__ void unit_segment(F3 origin, F3 endpoint, F3 expected
 // Checked products (frexp / scalbn forms)
 // ------------------------------------------------------------------------------------------------
 
+// The factors of one product, passed by value so that they stay in registers.
+template <int NN, int ND>
+struct Factors {
+    float num[NN], den[ND];
+    __device__ __forceinline__ Factors(const float (&n)[NN], const float (&d)[ND]) {
+#pragma unroll
+        for (int i = 0; i < NN; ++i) {
+            num[i] = n[i];
+        }
+#pragma unroll
+        for (int i = 0; i < ND; ++i) {
+            den[i] = d[i];
+        }
+    }
+};
+
 // DirectLighting.hpp:21-62
 template <int NN, int ND>
-__device__ __forceinline__ float checked_product_quotient(const float (&num)[NN], const float (&den)[ND],
-                                                          Lane& lane) {
+BF_BLOCK float factors_quotient(const Factors<NN, ND> f, Lane& lane) {
     float significand = 1.0F;
     int exponent = 0;
 #pragma unroll
     for (int i = 0; i < NN; ++i) {
-        const float v = num[i];
+        const float v = f.num[i];
         if (!isfinite(v) || v < 0.0F) {
             lane.fail();
             return 0.0F;
@@ -361,7 +395,7 @@ __device__ __forceinline__ float checked_product_quotient(const float (&num)[NN]
     }
 #pragma unroll
     for (int i = 0; i < ND; ++i) {
-        const float v = den[i];
+        const float v = f.den[i];
         if (!isfinite(v) || !(v > 0.0F)) {
             lane.fail();
             return 0.0F;
@@ -379,22 +413,26 @@ __device__ __forceinline__ float checked_product_quotient(const float (&num)[NN]
     return result;
 }
 
+template <int NN, int ND>
+__device__ __forceinline__ float checked_product_quotient(const float (&num)[NN], const float (&den)[ND], Lane& lane) {
+    return factors_quotient(Factors<NN, ND>(num, den), lane);
+}
+
 // RoughDielectric.hpp:52-86
 template <int NN, int ND>
-__device__ __forceinline__ float checked_product_ratio(const float (&num)[NN], const float (&den)[ND],
-                                                       Lane& lane) {
+BF_BLOCK float factors_ratio(const Factors<NN, ND> f, Lane& lane) {
     bool zero = false;
 #pragma unroll
     for (int i = 0; i < NN; ++i) {
-        if (!isfinite(num[i]) || num[i] < 0.0F) {
+        if (!isfinite(f.num[i]) || f.num[i] < 0.0F) {
             lane.fail();
             return 0.0F;
         }
-        zero = zero || num[i] == 0.0F;
+        zero = zero || f.num[i] == 0.0F;
     }
 #pragma unroll
     for (int i = 0; i < ND; ++i) {
-        if (!isfinite(den[i]) || !(den[i] > 0.0F)) {
+        if (!isfinite(f.den[i]) || !(f.den[i] > 0.0F)) {
             lane.fail();
             return 0.0F;
         }
@@ -407,14 +445,14 @@ __device__ __forceinline__ float checked_product_ratio(const float (&num)[NN], c
 #pragma unroll
     for (int i = 0; i < NN; ++i) {
         int ve = 0, ne = 0;
-        const float vs = frexpf(num[i], &ve);
+        const float vs = frexpf(f.num[i], &ve);
         significand = frexpf(significand * vs, &ne);
         exponent += ve + ne;
     }
 #pragma unroll
     for (int i = 0; i < ND; ++i) {
         int ve = 0, ne = 0;
-        const float vs = frexpf(den[i], &ve);
+        const float vs = frexpf(f.den[i], &ve);
         significand = frexpf(significand / vs, &ne);
         exponent += ne - ve;
     }
@@ -423,6 +461,11 @@ __device__ __forceinline__ float checked_product_ratio(const float (&num)[NN], c
         lane.fail();
     }
     return result;
+}
+
+template <int NN, int ND>
+__device__ __forceinline__ float checked_product_ratio(const float (&num)[NN], const float (&den)[ND], Lane& lane) {
+    return factors_ratio(Factors<NN, ND>(num, den), lane);
 }
 
 // MisHeuristics.hpp:142-172
@@ -621,7 +664,7 @@ struct Smith {
 };
 
 // GgxMicrofacet.hpp:134-184
-__device__ __forceinline__ Smith smith_terms(float ax, float ay, F3 w, Lane& lane) {
+BF_BLOCK Smith smith_terms(float ax, float ay, F3 w, Lane& lane) {
     Smith t;
     if (ax == ay) {
         const float sine = hypot2f(w.x, w.y);
@@ -651,7 +694,7 @@ __device__ __forceinline__ Smith smith_terms(float ax, float ay, F3 w, Lane& lan
 }
 
 // GgxMicrofacet.hpp:232-270
-__device__ __forceinline__ float ggx_d(float ax, float ay, F3 m, Lane& lane) {
+BF_BLOCK float ggx_d(float ax, float ay, F3 m, Lane& lane) {
     if (!unit_length(m)) {
         lane.fail();
         return 0.0F;
@@ -704,7 +747,7 @@ __device__ __forceinline__ float ggx_g2(float ax, float ay, F3 wo, F3 wi, Lane& 
 }
 
 // GgxMicrofacet.hpp:355-388
-__device__ __forceinline__ float ggx_vndf_pdf(float ax, float ay, F3 wo, F3 m, Lane& lane) {
+BF_BLOCK float ggx_vndf_pdf(float ax, float ay, F3 wo, F3 m, Lane& lane) {
     if (!unit_length(wo) || !unit_length(m)) {
         lane.fail();
         return 0.0F;
@@ -727,7 +770,7 @@ __device__ __forceinline__ float ggx_vndf_pdf(float ax, float ay, F3 wo, F3 m, L
 }
 
 // GgxMicrofacet.hpp:71-103
-__device__ __forceinline__ F3 ggx_normalize(F3 v, Lane& lane) {
+BF_BLOCK F3 ggx_normalize(F3 v, Lane& lane) {
     const float length = hypot2f(hypot2f(v.x, v.y), v.z);
     if (!isfinite(length) || !(length > 0.0F)) {
         lane.fail();
@@ -753,7 +796,7 @@ __device__ __forceinline__ float nonnegative_roundoff(float value, float scale, 
 }
 
 // GgxMicrofacet.hpp:390-525
-static __device__ bool ggx_sample_vndf(float ax, float ay, F3 wo, float u, float v, F3& m_out, Lane& lane) {
+BF_SHARED bool ggx_sample_vndf(float ax, float ay, F3 wo, float u, float v, F3& m_out, Lane& lane) {
     if (!unit_length(wo)) {
         lane.fail();
         return false;
@@ -823,7 +866,7 @@ static __device__ bool ggx_sample_vndf(float ax, float ay, F3 wo, float u, float
 }
 
 // Fresnel.hpp:27-104
-__device__ __forceinline__ float squared_magnitude_ratio(float nr, float ni, float dr, float di, Lane& lane) {
+BF_BLOCK float squared_magnitude_ratio(float nr, float ni, float dr, float di, Lane& lane) {
     const float n = hypot2f(nr, ni);
     const float d = hypot2f(dr, di);
     if (!isfinite(n) || !isfinite(d) || !(d > 0.0F)) {
@@ -838,10 +881,7 @@ __device__ __forceinline__ float squared_magnitude_ratio(float nr, float ni, flo
     return r;
 }
 
-// Out of line, as is dielectric_fresnel: each is called per packet lane from several evaluation
-// sites, and inlined copies made the shading kernels stall on instruction fetch (measured: shading
-// 4 % faster on the BVH-stress frame out of line).
-static __device__ __noinline__ float conductor_fresnel_lane(float cosine, float eta, float k, Lane& lane) {
+BF_SHARED float conductor_fresnel_lane(float cosine, float eta, float k, Lane& lane) {
     if (eta == 1.0F && k == 0.0F) {
         return 0.0F;
     }
@@ -889,7 +929,7 @@ static __device__ __noinline__ float conductor_fresnel_lane(float cosine, float 
 }
 
 // Fresnel.hpp:107-170
-static __device__ __noinline__ float dielectric_fresnel(float cosine, float eta_i, float eta_t, Lane& lane) {
+BF_SHARED float dielectric_fresnel(float cosine, float eta_i, float eta_t, Lane& lane) {
     if (!isfinite(cosine) || cosine < 0.0F || cosine > 1.0F) {
         lane.fail();
         return 1.0F;
@@ -936,7 +976,7 @@ static __device__ __noinline__ float dielectric_fresnel(float cosine, float eta_
 }
 
 // RoughConductorReflection.hpp:68-106 / RoughDielectric.hpp:136-170
-__device__ __forceinline__ void half_vector_geometry(F3 wo, F3 wi, F3& m, float& half_cos, Lane& lane) {
+BF_BLOCK void half_vector_geometry(F3 wo, F3 wi, F3& m, float& half_cos, Lane& lane) {
     const F3 h{wo.x + wi.x, wo.y + wi.y, wo.z + wi.z};
     const float length = hypot2f(hypot2f(h.x, h.y), h.z);
     if (!isfinite(length) || !(length > 0.0F)) {
@@ -956,7 +996,7 @@ __device__ __forceinline__ void half_vector_geometry(F3 wo, F3 wi, F3& m, float&
 }
 
 // RoughConductorReflection.hpp:167-238
-static __device__ void conductor_eval(const ClosureData& c, F3 wo, F3 wi, float (&out)[4], Lane& lane) {
+BF_SHARED void conductor_eval(const ClosureData& c, F3 wo, F3 wi, float (&out)[4], Lane& lane) {
     out[0] = out[1] = out[2] = out[3] = 0.0F;
     if (!unit_length(wo) || !unit_length(wi)) {
         lane.fail();
@@ -990,7 +1030,7 @@ static __device__ void conductor_eval(const ClosureData& c, F3 wo, F3 wi, float 
     }
 }
 
-static __device__ float conductor_pdf(const ClosureData& c, F3 wo, F3 wi, Lane& lane) {
+BF_SHARED float conductor_pdf(const ClosureData& c, F3 wo, F3 wi, Lane& lane) {
     if (!unit_length(wo) || !unit_length(wi)) {
         lane.fail();
         return 0.0F;
@@ -1034,7 +1074,7 @@ struct TransmissionGeometry {
 };
 
 // RoughDielectric.hpp:172-223
-static __device__ TransmissionGeometry transmission_geometry(F3 of, F3 inf, const Interface& f, Lane& lane) {
+BF_BLOCK TransmissionGeometry transmission_geometry(F3 of, F3 inf, const Interface& f, Lane& lane) {
     TransmissionGeometry g{};
     g.valid = false;
     F3 h{fmaf(f.nie, of.x, f.nte * inf.x), fmaf(f.nie, of.y, f.nte * inf.y), fmaf(f.nie, of.z, f.nte * inf.z)};
@@ -1085,7 +1125,7 @@ __device__ __forceinline__ void scale_spectrum(const float (&c)[4], float scale,
 }
 
 // RoughDielectric.hpp:299-381 (radiance mode)
-static __device__ void dielectric_eval(const ClosureData& c, F3 wo, F3 wi, float (&out)[4], Lane& lane) {
+BF_SHARED void dielectric_eval(const ClosureData& c, F3 wo, F3 wi, float (&out)[4], Lane& lane) {
     out[0] = out[1] = out[2] = out[3] = 0.0F;
     if (!unit_length(wo) || !unit_length(wi)) {
         lane.fail();
@@ -1131,7 +1171,7 @@ static __device__ void dielectric_eval(const ClosureData& c, F3 wo, F3 wi, float
 }
 
 // RoughDielectric.hpp:383-467
-static __device__ float dielectric_pdf(const ClosureData& c, F3 wo, F3 wi, Lane& lane) {
+BF_SHARED float dielectric_pdf(const ClosureData& c, F3 wo, F3 wi, Lane& lane) {
     if (!unit_length(wo) || !unit_length(wi)) {
         lane.fail();
         return 0.0F;
@@ -1250,7 +1290,7 @@ __device__ __forceinline__ bool cone_ratio(float numerator, float denominator, f
 
 // advance_ray_cone_to_hit: the cone carried from the ray origin to the hit at parameter t of a ray
 // whose direction d need not be unit (its length taken as max|d| * |d / max|d||).
-static __device__ bool cone_advance(float2 cone, F3 d, float t, float2& out) {
+BF_SHARED bool cone_advance(float2 cone, F3 d, float t, float2& out) {
     if (!cone_valid(cone) || !isfinite(t) || t < 0.0F) {
         return false;
     }
@@ -1583,12 +1623,12 @@ constexpr float kFonCoefficient = 0.5F - 2.0F * kInvPi / 3.0F;
 constexpr float kFonAverageCoefficient = 2.0F / 3.0F - 28.0F * kInvPi / 15.0F;
 constexpr float kFonAverageLossCoefficient = kFonCoefficient - kFonAverageCoefficient;
 
-static __device__ __noinline__ float atan2_f(float y, float x) {
+BF_SHARED float atan2_f(float y, float x) {
     return static_cast<float>(atan2(static_cast<double>(y), static_cast<double>(x)));
 }
 
 // directional_loss_shape: 1 - E_FON for unit albedo without the factor A_F * r
-static __device__ float eon_loss_shape(F3 d, Lane& lane) {
+BF_SHARED float eon_loss_shape(F3 d, Lane& lane) {
     const float sine = hypot2f(d.x, d.y);
     const float cosine = d.z;
     const float angle = atan2_f(sine, cosine);
@@ -1601,7 +1641,7 @@ static __device__ float eon_loss_shape(F3 d, Lane& lane) {
     return loss;
 }
 
-static __device__ void eon_eval(const ClosureData& c, F3 wo, F3 wi, float (&out)[4], Lane& lane) {
+BF_SHARED void eon_eval(const ClosureData& c, F3 wo, F3 wi, float (&out)[4], Lane& lane) {
     out[0] = out[1] = out[2] = out[3] = 0.0F;
     if (!unit_length(wo) || !unit_length(wi)) {
         lane.fail();
@@ -1692,7 +1732,7 @@ __device__ __forceinline__ float delta_squared_ratio(float num, float den, Lane&
     return result;
 }
 
-static __device__ void specular_sample(const ClosureData& c, F3 wo, BsdfSample& s, Lane& lane) {
+BF_SHARED void specular_sample(const ClosureData& c, F3 wo, BsdfSample& s, Lane& lane) {
     s.valid = false;
     s.delta = true;
     s.pdf = 1.0F;
@@ -1905,7 +1945,7 @@ __device__ __forceinline__ bool add_compensated(float value, float& sum, float& 
 }
 
 // build_component_distribution (ClosureMixture.hpp:122-234) for n >= 2 renormalised probabilities
-static __device__ bool component_distribution(const float* probabilities, uint32_t n, float* out_p, float* out_cdf) {
+BF_SHARED bool component_distribution(const float* probabilities, uint32_t n, float* out_p, float* out_cdf) {
 #pragma unroll
     for (uint32_t i = 0; i <= kMaxClosures; ++i) {
         out_cdf[i] = 0.0F;
@@ -1996,7 +2036,7 @@ __device__ __forceinline__ float positive_probability_product(float selection, f
 }
 
 // mix_probability_densities (ClosureMixture.hpp:270-334)
-static __device__ float mix_densities(const float* probabilities, const float* conditional, uint32_t n, Lane& lane) {
+BF_SHARED float mix_densities(const float* probabilities, const float* conditional, uint32_t n, Lane& lane) {
     float maximum = 0.0F;
     for (uint32_t i = 0; i < n; ++i) {
         if (!isfinite(conditional[i]) || conditional[i] < 0.0F) {
