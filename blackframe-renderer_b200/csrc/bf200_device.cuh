@@ -64,7 +64,8 @@ struct PunctualLight {
 struct SceneView {
     uint32_t instance_count;
     uint32_t light_count;
-    const float4* inst_world_box;  // padded world box per instance: lo (xyz, w = visibility mask bits), hi
+    const float4* inst_world_box;  // padded world box per instance: lo (xyz, w = visibility mask bits),
+                                   // hi (xyz, w = BLAS root node or leaf code bits)
     int32_t tlas_root;             // BVH4 over the instances' world boxes (leaves ~instance), or -1
     const float4* inst_to_object;  // 3 rows (m0..m3) per instance
     const float4* inst_to_world;   // 3 rows per instance
@@ -136,6 +137,9 @@ constexpr uint8_t kRouteNone = 0xFFU;  // slot not shaded this iteration / no sh
 constexpr uint32_t kCompactTile = 4096U;
 constexpr uint32_t kCompactMaxRoutes = kRouteCount;
 constexpr uint32_t kCompactFewRoutes = 4U;
+
+constexpr uint32_t kWavefrontCounters = 24U;
+constexpr uint32_t kCounterTraceCursor = 8U, kCounterOccludeCursor = 15U, kCounterTraced = 16U;
 
 // Slot states of the persistent wavefront.
 constexpr uint8_t kSlotEmpty = 0, kSlotActive = 1, kSlotDone = 2;
@@ -221,12 +225,14 @@ struct Wavefront {
     float4* shadow_d;   // direction
     float4* shadow_c;   // contribution (unoccluded)
     uint32_t* shadow_queue;    // slots with a shadow ray, in slot order
+    uint32_t* trace_queue;     // slots with a ray to trace (the shadow queue's memory, before shading)
     uint32_t* shadow_offsets;  // 2 queue boundaries
     uint32_t* tile_counts;     // compaction scratch: kCompactMaxRoutes x tiles
     // counters: [0] shadow queue size, [1] next path to claim, [2] active slots,
     //           [3] extension segments, [4] shadow segments, [5] failed lanes,
     //           [6] first failure path (min), [7] first failure code, [8] k_trace fetch cursor,
-    //           [9] iterations and [10] iteration-bound flag of a device-side loop
+    //           [9] iterations and [10] iteration-bound flag of a device-side loop, [11..14] the
+    //           cone-carrying kernels' stage counts, [15] k_occlude fetch cursor, [16] traced slots
     unsigned long long* counters;
 };
 

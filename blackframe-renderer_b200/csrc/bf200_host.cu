@@ -86,6 +86,7 @@ struct bf200_scene {
     // transform-only refit (bf200_scene_refit): what the instance level is rebuilt from
     uint64_t fingerprint = 0;           // the description without its instance transforms
     std::vector<float> object_boxes;    // per geometry: lo xyz, hi xyz
+    std::vector<uint32_t> blas_roots;   // per geometry: root node or leaf code
     uint32_t tlas_first = 0;            // first TLAS node in the node array (when there is a TLAS)
     std::vector<BvhNode4> tlas_nodes;   // host copy of the TLAS nodes
     uint32_t instance_triangles = 0;
@@ -956,13 +957,14 @@ size_t carve_wavefront(char* base, uint32_t capacity, Wavefront* out) {
     w.mask = reinterpret_cast<uint32_t*>(take(4 * n));
     w.route_queue = reinterpret_cast<uint32_t*>(take(4 * n));
     w.shadow_queue = reinterpret_cast<uint32_t*>(take(4 * n));
+    w.trace_queue = w.shadow_queue;
     w.state = reinterpret_cast<uint8_t*>(take(n));
     w.route = reinterpret_cast<uint8_t*>(take(n));
     w.shadow_key = reinterpret_cast<uint8_t*>(take(n));
     w.tile_counts = reinterpret_cast<uint32_t*>(take(4 * kCompactMaxRoutes * (tiles == 0 ? 1 : tiles)));
     w.route_offsets = reinterpret_cast<uint32_t*>(take(4 * (kRouteCount + 1)));
     w.shadow_offsets = reinterpret_cast<uint32_t*>(take(4 * 2));
-    w.counters = reinterpret_cast<unsigned long long*>(take(16 * sizeof(unsigned long long)));
+    w.counters = reinterpret_cast<unsigned long long*>(take(kWavefrontCounters * sizeof(unsigned long long)));
     if (out != nullptr) {
         *out = w;
     }
@@ -980,7 +982,7 @@ blackframe_status ensure_capacity(bf200_context* c) {
         return cuda_fail(c, e, "wavefront allocation");
     }
     carve_wavefront(static_cast<char*>(c->arena), n, &c->w);
-    e = cudaMallocHost(&c->pinned_counters, 16 * sizeof(unsigned long long));
+    e = cudaMallocHost(&c->pinned_counters, kWavefrontCounters * sizeof(unsigned long long));
     if (e != cudaSuccess) {
         return cuda_fail(c, e, "pinned counters");
     }
@@ -1118,7 +1120,7 @@ blackframe_status run_wavefront_graph(bf200_context* c, const bf200_scene* s, Pa
     cudaStream_t st = c->stream;
     cudaError_t e = cudaMemsetAsync(w.state, 0, w.capacity, st);
     if (e == cudaSuccess) {
-        e = cudaMemsetAsync(w.counters, 0, 16 * sizeof(unsigned long long), st);
+        e = cudaMemsetAsync(w.counters, 0, kWavefrontCounters * sizeof(unsigned long long), st);
     }
     if (e == cudaSuccess) {  // counters[6], the first failing path, is a minimum
         e = cudaMemsetAsync(w.counters + 6, 0xFF, sizeof(unsigned long long), st);
@@ -1173,7 +1175,7 @@ blackframe_status run_wavefront_graph(bf200_context* c, const bf200_scene* s, Pa
         e = launch_retire(w, src, grid, st);
     }
     if (e == cudaSuccess) {
-        e = cudaMemcpyAsync(c->pinned_counters, w.counters, 16 * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
+        e = cudaMemcpyAsync(c->pinned_counters, w.counters, kWavefrontCounters * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
                             st);
     }
     if (e == cudaSuccess) {
@@ -1227,7 +1229,7 @@ blackframe_status run_wavefront(bf200_context* c, const bf200_scene* s, PathSour
     cudaStream_t st = c->stream;
     cudaError_t e = cudaMemsetAsync(w.state, 0, w.capacity, st);
     if (e == cudaSuccess) {
-        e = cudaMemsetAsync(w.counters, 0, 16 * sizeof(unsigned long long), st);
+        e = cudaMemsetAsync(w.counters, 0, kWavefrontCounters * sizeof(unsigned long long), st);
     }
     if (e != cudaSuccess) {
         return cuda_fail(c, e, "wavefront reset");
@@ -1299,7 +1301,7 @@ blackframe_status run_wavefront(bf200_context* c, const bf200_scene* s, PathSour
     e = launch_retire(w, src, grid, st);
     ++launches;
     if (e == cudaSuccess) {
-        e = cudaMemcpyAsync(c->pinned_counters, w.counters, 16 * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
+        e = cudaMemcpyAsync(c->pinned_counters, w.counters, kWavefrontCounters * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
                             st);
     }
     cudaEventRecord(stop, st);
@@ -1597,6 +1599,9 @@ BF200_EXPORT blackframe_status bf200_scene_create(bf200_context* c, const bf200_
                 object_box[g].grow(d->positions + 3ULL * (geom.vertex_offset + local[t]));
             }
         }
+        for (const uint4& g : geom_info) {
+            scene->blas_roots.push_back(g.z);
+        }
         const auto t_instances = Clock::now();
         // instance ranges on the traversal stack carry 14-bit first indices
         if (d->instance_count >= (1U << 14)) {
@@ -1644,6 +1649,7 @@ BF200_EXPORT blackframe_status bf200_scene_create(bf200_context* c, const bf200_
             world_box[2ULL * i] = make_float4(b.lo[0], b.lo[1], b.lo[2], 0.0F);
             std::memcpy(&world_box[2ULL * i].w, &d->instances[i].visibility_mask, 4);  // mask bits, not a number
             world_box[2ULL * i + 1] = make_float4(b.hi[0], b.hi[1], b.hi[2], 0.0F);
+            std::memcpy(&world_box[2ULL * i + 1].w, &geom_info[d->instances[i].geometry_index].z, 4);  // root code
         }
         scene->node_count = nodes4.size();
         scene->triangle_count = leaf_tris.size() / 3;
@@ -1967,6 +1973,7 @@ BF200_EXPORT blackframe_status bf200_scene_refit(bf200_scene* s, const bf200_sce
             world_box[2ULL * i] = make_float4(boxes[i].lo[0], boxes[i].lo[1], boxes[i].lo[2], 0.0F);
             std::memcpy(&world_box[2ULL * i].w, &inst.visibility_mask, 4);  // mask bits, not a number
             world_box[2ULL * i + 1] = make_float4(boxes[i].hi[0], boxes[i].hi[1], boxes[i].hi[2], 0.0F);
+            std::memcpy(&world_box[2ULL * i + 1].w, &s->blas_roots[inst.geometry_index], 4);  // root code
         }
         if (lights.size() != s->light_count || light_areas.size() != s->light_triangles) {
             return fail(c, BLACKFRAME_STATUS_EXTENSION_FAILURE, "internal error: refit changed the light layout");
@@ -2464,7 +2471,7 @@ blackframe_status run_wavefront_noalloc(bf200_context* c, const bf200_scene* s, 
     // (counters[6], a minimum) starts at all ones
     cudaError_t e = cudaMemsetAsync(w.state, 0, w.capacity, st);
     if (e == cudaSuccess) {
-        e = cudaMemsetAsync(w.counters, 0, 8 * sizeof(unsigned long long), st);
+        e = cudaMemsetAsync(w.counters, 0, kWavefrontCounters * sizeof(unsigned long long), st);
     }
     if (e == cudaSuccess) {
         e = cudaMemsetAsync(w.counters + 6, 0xFF, sizeof(unsigned long long), st);
@@ -3043,7 +3050,7 @@ cudaError_t lane_start_chunk(const bf200_film_job_v1& job, LaneState& lane, cuda
     lane.phase = 1;
     cudaError_t e = cudaMemsetAsync(lane.w.state, 0, lane.w.capacity, st);
     if (e == cudaSuccess) {
-        e = cudaMemsetAsync(lane.w.counters, 0, 8 * sizeof(unsigned long long), st);
+        e = cudaMemsetAsync(lane.w.counters, 0, kWavefrontCounters * sizeof(unsigned long long), st);
     }
     if (e == cudaSuccess) {  // counters[6], the first failing path, is a minimum
         e = cudaMemsetAsync(lane.w.counters + 6, 0xFF, sizeof(unsigned long long), st);

@@ -11,7 +11,7 @@ namespace bf200 {
 
 cudaError_t launch_world_normals(const SceneView& s, uint32_t total, float4* out, uint32_t* failures,
                                  cudaStream_t stream);
-// stage 0: k_regenerate; 1: k_trace; 2: route compaction, the per-route k_shade kernels, shadow
+// stage 0: k_regenerate; 1: k_trace, k_hits; 2: route compaction, the per-route k_shade kernels, shadow
 // compaction; 3: k_occlude. Adds the number of kernels launched to *launches. With `adjoint`, the
 // shading and occlusion stages run as the path-replay adjoint's replay.
 cudaError_t launch_stage(int stage, const SceneView& s, const Wavefront& w, const PathSource& src,

@@ -5,7 +5,8 @@
 //   k_regenerate : path retirement and regeneration with device camera rays (seed/camera stages,
 //                  CudaWavefrontStages.cu:1269-1406)
 //   k_trace      : scene_closest_hit_kernel + classify/miss stages (CudaSceneClosestHit.cu:1199,
-//                  CudaWavefrontStages.cu:1434, :3962); writes each slot's shading route
+//                  CudaWavefrontStages.cu:1434, :3962), in bf200_pool.cuh; k_hits completes the hits
+//                  and writes each slot's shading route
 //   k_shade<K>   : shade_stage_kernel (CudaWavefrontStages.cu:4107-4727), one instantiation per
 //                  closure kind over that route's queue (bf200_compact.cu builds the queues)
 //   k_occlude    : scene_occlusion_kernel + process_shadow_kernel (CudaSceneClosestHit.cu:1243,
@@ -20,6 +21,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <climits>
 
 #include "bf200_device.cuh"
@@ -28,14 +30,8 @@
 #include "bf200_light_tree_device.cuh"
 
 // Resident 256-thread blocks per SM the register allocation must allow, per stage kernel.
-#ifndef BF200_INTERSECT_MIN_BLOCKS
-#define BF200_INTERSECT_MIN_BLOCKS 2
-#endif
 #ifndef BF200_SHADE_MIN_BLOCKS
 #define BF200_SHADE_MIN_BLOCKS 2
-#endif
-#ifndef BF200_OCCLUDE_MIN_BLOCKS
-#define BF200_OCCLUDE_MIN_BLOCKS 2
 #endif
 
 namespace bf200 {
@@ -197,8 +193,23 @@ __device__ __forceinline__ int slow_path(float4 v0, float4 v1, float4 v2, F3 o, 
     return r.code;
 }
 
-// The float nearest to num/den when a forward error bound proves it; otherwise NaN.
+// The float nearest to num/den when a forward error bound proves it; otherwise NaN. Bounds below 2^-46
+// of their values, the usual case, leave the quotient within 2^-44 of its own size: one division
+// decides, and an interval that rounds to one float holds the same float as the narrower one of the
+// general case.
+static __device__ __noinline__ float certain_round_general(double num, double num_bound, double den, double den_bound);
 __device__ __forceinline__ float certain_round(double num, double num_bound, double den, double den_bound) {
+    if (num_bound <= fabs(num) * 0x1p-46 && den_bound <= fabs(den) * 0x1p-46) {
+        const double q = num / den;
+        const double slack = fabs(q) * 0x1p-44;
+        const float lo = __double2float_rn(q - slack), hi = __double2float_rn(q + slack);
+        if (lo == hi && q != 0.0) {
+            return lo;
+        }
+    }
+    return certain_round_general(num, num_bound, den, den_bound);
+}
+static __device__ __noinline__ float certain_round_general(double num, double num_bound, double den, double den_bound) {
     if (!(fabs(num) > 2.0 * num_bound) || !(fabs(den) > 2.0 * den_bound)) {
         return __int_as_float(0x7fc00000);
     }
@@ -331,18 +342,14 @@ constexpr float kSlackHi = 1.0F + 2.0F * kGamma3;
 struct RayInv {
     F3 o;
     F3 inv;
-    bool px, py, pz;  // axis-parallel components
-    bool parallel;    // any of them
+    uint32_t axes;  // axis-parallel components: bit 0 x, 1 y, 2 z
 };
 
 __device__ __forceinline__ RayInv make_ray_inv(F3 o, F3 d) {
     RayInv r;
     r.o = o;
-    r.px = d.x == 0.0F;
-    r.py = d.y == 0.0F;
-    r.pz = d.z == 0.0F;
-    r.inv = F3{r.px ? 0.0F : 1.0F / d.x, r.py ? 0.0F : 1.0F / d.y, r.pz ? 0.0F : 1.0F / d.z};
-    r.parallel = r.px || r.py || r.pz;
+    r.axes = (d.x == 0.0F ? 1U : 0U) | (d.y == 0.0F ? 2U : 0U) | (d.z == 0.0F ? 4U : 0U);
+    r.inv = F3{d.x == 0.0F ? 0.0F : 1.0F / d.x, d.y == 0.0F ? 0.0F : 1.0F / d.y, d.z == 0.0F ? 0.0F : 1.0F / d.z};
     return r;
 }
 
@@ -350,94 +357,62 @@ __device__ __forceinline__ RayInv make_ray_inv(F3 o, F3 d) {
 // in [t_min, t_max] (each computed slab parameter is within a relative gamma(3) of the exact one,
 // and its sign is exact). A ray with no axis-parallel component takes the first branch, where the
 // slack factors scale the largest entry and smallest exit parameter once: rounding a product with
-// a positive factor is monotonic, so that equals scaling each axis's parameter first.
-__device__ __forceinline__ bool slab(const RayInv& r, float lox, float hix, float loy, float hiy, float loz, float hiz,
-                                     float t_min, float t_max, float& near_out) {
-    if (!r.parallel) {
-        const float ax = (lox - r.o.x) * r.inv.x, bx = (hix - r.o.x) * r.inv.x;
-        const float ay = (loy - r.o.y) * r.inv.y, by = (hiy - r.o.y) * r.inv.y;
-        const float az = (loz - r.o.z) * r.inv.z, bz = (hiz - r.o.z) * r.inv.z;
-        const float entry = fmaxf(fmaxf(fminf(ax, bx), fminf(ay, by)), fminf(az, bz));
-        const float exit = fminf(fminf(fmaxf(ax, bx), fmaxf(ay, by)), fmaxf(az, bz));
-        const float near = fmaxf(t_min, entry * kSlackLo);
-        near_out = near;
-        return near <= fminf(t_max, exit * kSlackHi);
-    }
+// a positive factor is monotonic, so that equals scaling each axis's parameter first. Axis-parallel
+// rays are rare and take a shared copy, which keeps the four tests of a node visit short.
+static __device__ __noinline__ float2 slab_parallel(F3 o, F3 inv, uint32_t axes, float lox, float hix, float loy,
+                                                    float hiy, float loz, float hiz, float t_min, float t_max) {
     float near = t_min, far = t_max;
     bool inside = true;
-    if (r.px) {
-        inside = inside && lox <= r.o.x && r.o.x <= hix;
+    if ((axes & 1U) != 0U) {
+        inside = inside && lox <= o.x && o.x <= hix;
     } else {
-        const float a = (lox - r.o.x) * r.inv.x, b = (hix - r.o.x) * r.inv.x;
+        const float a = (lox - o.x) * inv.x, b = (hix - o.x) * inv.x;
         near = fmaxf(near, fminf(a, b) * kSlackLo);
         far = fminf(far, fmaxf(a, b) * kSlackHi);
     }
-    if (r.py) {
-        inside = inside && loy <= r.o.y && r.o.y <= hiy;
+    if ((axes & 2U) != 0U) {
+        inside = inside && loy <= o.y && o.y <= hiy;
     } else {
-        const float a = (loy - r.o.y) * r.inv.y, b = (hiy - r.o.y) * r.inv.y;
+        const float a = (loy - o.y) * inv.y, b = (hiy - o.y) * inv.y;
         near = fmaxf(near, fminf(a, b) * kSlackLo);
         far = fminf(far, fmaxf(a, b) * kSlackHi);
     }
-    if (r.pz) {
-        inside = inside && loz <= r.o.z && r.o.z <= hiz;
+    if ((axes & 4U) != 0U) {
+        inside = inside && loz <= o.z && o.z <= hiz;
     } else {
-        const float a = (loz - r.o.z) * r.inv.z, b = (hiz - r.o.z) * r.inv.z;
+        const float a = (loz - o.z) * inv.z, b = (hiz - o.z) * inv.z;
         near = fmaxf(near, fminf(a, b) * kSlackLo);
         far = fminf(far, fmaxf(a, b) * kSlackHi);
     }
+    return make_float2(near, inside && near <= far ? 1.0F : 0.0F);
+}
+
+__device__ __forceinline__ bool slab(const RayInv& r, float lox, float hix, float loy, float hiy, float loz, float hiz,
+                                     float t_min, float t_max, float& near_out) {
+    if (r.axes != 0U) {
+        const float2 v = slab_parallel(r.o, r.inv, r.axes, lox, hix, loy, hiy, loz, hiz, t_min, t_max);
+        near_out = v.x;
+        return v.y != 0.0F;
+    }
+    const float ax = (lox - r.o.x) * r.inv.x, bx = (hix - r.o.x) * r.inv.x;
+    const float ay = (loy - r.o.y) * r.inv.y, by = (hiy - r.o.y) * r.inv.y;
+    const float az = (loz - r.o.z) * r.inv.z, bz = (hiz - r.o.z) * r.inv.z;
+    const float entry = fmaxf(fmaxf(fminf(ax, bx), fminf(ay, by)), fminf(az, bz));
+    const float exit = fminf(fminf(fmaxf(ax, bx), fmaxf(ay, by)), fmaxf(az, bz));
+    const float near = fmaxf(t_min, entry * kSlackLo);
     near_out = near;
-    return inside && near <= far;
+    return near <= fminf(t_max, exit * kSlackHi);
 }
 
 // The slack factors only widen positive parameters; a negative lower bound is harmless because
 // t_min >= 0 clamps it, and a negative upper bound means the box is entirely behind the origin.
 
-// Traversal stack of one thread. The first kSharedStackEntries entries live in shared memory in
-// thread-interleaved columns (entry k of thread t at k * blockDim.x + t: every lane of a warp hits
-// its own bank at any depth); deeper entries, which the shallow BVHs of small scenes never reach,
-// go to a local array.
-constexpr int kSharedStackEntries = 32;
-
-struct TraversalStack {
-    int* column;
-    uint32_t stride;
-    int deep[kTraversalStack - kSharedStackEntries];
-    __device__ __forceinline__ void set(int sp, int v) {
-        if (sp < kSharedStackEntries) {
-            column[sp * stride] = v;
-        } else {
-            deep[sp - kSharedStackEntries] = v;
-        }
-    }
-    __device__ __forceinline__ int get(int sp) const {
-        return sp < kSharedStackEntries ? column[sp * stride] : deep[sp - kSharedStackEntries];
-    }
-};
-
-__device__ __forceinline__ TraversalStack thread_stack(int* shared) {
-    TraversalStack st;
-    st.column = shared + threadIdx.x;
-    st.stride = blockDim.x;
-    return st;
-}
-
 struct ClosestResult {
     float t;
-    uint32_t instance, primitive;
+    uint32_t instance;
     uint32_t leaf;  // leaf triangle index of the winner
     bool failed;
 };
-
-__device__ __forceinline__ bool precedes(float t, uint32_t inst, uint32_t prim, const ClosestResult& best) {
-    if (t != best.t) {
-        return t < best.t;
-    }
-    if (inst != best.instance) {
-        return inst < best.instance;
-    }
-    return prim < best.primitive;
-}
 
 // Children of a BVH4 node whose boxes the ray meets within [t_min, limit], ordered near to far
 // (a five-comparator sorting network on fixed slots, so everything stays in registers); returns
@@ -504,282 +479,10 @@ __device__ __forceinline__ int tlas_entry(int node) {
     return kInstanceEntry + static_cast<int>(kTlasFlag | static_cast<uint32_t>(node));
 }
 
-// Starts a walk's stack. With few instances every visible instance whose world box the ray meets
-// within [t_min, t_max] goes on as a one-instance range, the lowest index on top, with the warp in
-// step; otherwise the TLAS root goes on and the instance boxes are met through it.
-__device__ __forceinline__ void push_instances(const SceneView& s, const RayInv& world, float t_min, float t_max,
-                                               uint32_t mask, TraversalStack& stack, int& sp) {
-    if (s.tlas_root >= 0) {
-        stack.set(sp++, tlas_entry(s.tlas_root));
-        return;
-    }
-    for (int inst = static_cast<int>(s.instance_count) - 1; inst >= 0; --inst) {
-        const float4 blo = s.inst_world_box[2 * inst], bhi = s.inst_world_box[2 * inst + 1];
-        float near;
-        if ((mask & __float_as_uint(blo.w)) == 0U ||
-            !slab(world, blo.x, bhi.x, blo.y, bhi.y, blo.z, bhi.z, t_min, t_max, near)) {
-            continue;
-        }
-        stack.set(sp++, instance_range(static_cast<uint32_t>(inst), 1U));
-    }
-}
-
-// Pushes the children a node visit returned, the farthest first so that the nearest comes next.
-// Children of a TLAS node go on as TLAS entries (nodes) and one-instance ranges (instance leaves).
-__device__ __forceinline__ void push_children(const int (&kids)[4], int count, bool tlas, TraversalStack& stack,
-                                              int& sp, bool& failed) {
-#pragma unroll
-    for (int k = 3; k >= 0; --k) {
-        if (k < count) {
-            if (sp < kTraversalStack) {
-                const int kid = kids[k];
-                stack.set(sp++, !tlas ? kid
-                                      : kid >= 0 ? tlas_entry(kid) : instance_range(static_cast<uint32_t>(~kid), 1U));
-            } else {
-                failed = true;
-            }
-        }
-    }
-}
-
-// An instance range (code = first << 15 | count) yields its first instance: false when the ray's
-// visibility mask excludes it or its world box is not met within [t_min, limit]; otherwise the ray
-// moves into its object space, its BLAS root goes on above the rest of the range, and the call
-// returns true.
-__device__ __forceinline__ bool enter_instance(const SceneView& s, uint32_t code, const RayInv& world, F3 o, F3 d,
-                                               float t_min, float limit, uint32_t mask, TraversalStack& stack,
-                                               int& sp, bool& failed, uint32_t& inst_out, F3& ro, F3& rd,
-                                               RayInv& r) {
-    const uint32_t inst = code >> kInstanceBits, count = code & ((1U << kInstanceBits) - 1U);
-    if (count > 1U) {
-        stack.set(sp++, instance_range(inst + 1U, count - 1U));
-    }
-    const float4 blo = s.inst_world_box[2ULL * inst], bhi = s.inst_world_box[2ULL * inst + 1];
-    float near;
-    if ((mask & __float_as_uint(blo.w)) == 0U ||
-        !slab(world, blo.x, bhi.x, blo.y, bhi.y, blo.z, bhi.z, t_min, limit, near)) {
-        return false;
-    }
-    if (sp >= kTraversalStack) {
-        failed = true;
-        return false;
-    }
-    inst_out = inst;
-    const float4* m = s.inst_to_object + 3ULL * inst;
-    ro = xform_point(m, o);
-    rd = xform_vector(m, d);
-    r = make_ray_inv(ro, rd);
-    stack.set(sp++, static_cast<int>(s.geom_info[s.inst_info[inst].x].z));
-    return true;
-}
-
 // A sphere leaf's outcome codes are the triangle test's, so the walks treat both alike.
 static_assert(int(kSphereMiss) == int(kTriMiss) && int(kSphereHit) == int(kTriHit) &&
                   int(kSphereFailure) == int(kTriFailure),
               "outcome codes");
-
-// Per-lane walk state shared by the two traversals.
-struct Walk {
-    RayInv r;       // current ray (object space of the current instance)
-    F3 ro, rd;
-    uint32_t inst;  // current instance
-    int sp;
-    bool failed;
-};
-
-// Advances the walk until this lane holds a leaf (returned, in [-2^30, 0)) or its stack is empty
-// (returns 0). TLAS and BLAS nodes share one visit (with the world or the object-space ray), so
-// lanes at either level run it together; instance ranges are entered by enter_instance. Children
-// are pushed far first, so the nearer one comes next.
-__device__ __forceinline__ int next_leaf(const SceneView& s, const RayInv& world, F3 o, F3 d, float t_min,
-                                         float limit, uint32_t mask, TraversalStack& stack, Walk& w) {
-    while (w.sp > 0) {
-        const int entry = stack.get(--w.sp);
-        const uint32_t code = static_cast<uint32_t>(entry) ^ 0x80000000U;
-        const bool instance_level = entry < kLeafEntryMin;
-        if (instance_level && (code & kTlasFlag) == 0U) {
-            enter_instance(s, code, world, o, d, t_min, limit, mask, stack, w.sp, w.failed, w.inst, w.ro, w.rd, w.r);
-            continue;
-        }
-        if (!instance_level && entry < 0) {
-            return entry;
-        }
-        const int node = instance_level ? static_cast<int>(code & (kTlasFlag - 1U)) : entry;
-        int kids[4];
-        const int count = hit_children(instance_level ? world : w.r, s.nodes[node], t_min, limit, kids);
-        push_children(kids, count, instance_level, stack, w.sp, w.failed);
-    }
-    return 0;
-}
-
-// Closest-hit walk of one ray, in steps. closest_begin pushes the instance entries; each
-// closest_step advances the lane through nodes and instance entries to its next leaf ("while-
-// while": the warp reconverges before the leaf) and runs the exact triangle tests of that leaf;
-// it returns false once the ray's stack is empty. Ties keep the hit that comes first in
-// (instance, primitive) order, as the analytic accel's in-order scan does; boxes are culled only
-// when they start strictly beyond the current closest t, so neither the order nor the culling
-// changes the winner.
-struct ClosestWalk {
-    F3 o, d;
-    float t_min, t_max;
-    uint32_t mask;
-    RayInv world;
-    Walk w;
-    ClosestResult best;
-    bool found;
-};
-
-__device__ __forceinline__ void closest_begin(const SceneView& s, F3 o, F3 d, float t_min, float t_max,
-                                              uint32_t mask, TraversalStack& stack, ClosestWalk& c) {
-    c.o = o;
-    c.d = d;
-    c.t_min = t_min;
-    c.t_max = t_max;
-    c.mask = mask;
-    c.world = make_ray_inv(o, d);
-    c.w = Walk{c.world, o, d, 0xFFFFFFFFU, 0, false};
-    c.best.t = t_max;
-    c.best.instance = 0xFFFFFFFFU;
-    c.best.primitive = 0xFFFFFFFFU;
-    c.best.leaf = 0xFFFFFFFFU;
-    c.best.failed = false;
-    c.found = false;
-    push_instances(s, c.world, t_min, t_max, mask, stack, c.w.sp);
-}
-
-// SPH: the scene has analytic spheres (the walks of triangle-only scenes carry no sphere code).
-template <bool SPH>
-__device__ __forceinline__ bool closest_step(const SceneView& s, TraversalStack& stack, ClosestWalk& c) {
-    const int leaf_code =
-        next_leaf(s, c.world, c.o, c.d, c.t_min, c.found ? c.best.t : c.t_max, c.mask, stack, c.w);
-    if (leaf_code == 0) {
-        return false;
-    }
-    const uint32_t packed = static_cast<uint32_t>(~leaf_code);
-    const uint32_t first = packed >> kLeafCountBits;
-    const uint32_t n = (packed & (kMaxLeafSize - 1)) + 1U;
-    if (SPH && n == kSphereLeafCount) {  // an analytic sphere: one record, tested apart from the triangle loop
-        const float4 v0 = s.leaf_tris[3ULL * first];
-        const SphereHit h = sphere_intersect(v0, s.leaf_tris[3ULL * first + 1].x, c.w.ro, c.w.rd, c.t_min,
-                                             c.found ? c.best.t : c.t_max);
-        const uint32_t prim = __float_as_uint(v0.w);
-        if (h.outcome == kSphereFailure) {
-            c.w.failed = true;
-        } else if (h.outcome == kSphereHit && (!c.found || precedes(h.t, c.w.inst, prim, c.best))) {
-            c.best.t = h.t;
-            c.best.instance = c.w.inst;
-            c.best.primitive = prim;
-            c.best.leaf = first;
-            c.found = true;
-        }
-        return true;
-    }
-    for (uint32_t j = 0; j < n; ++j) {
-        const uint32_t leaf = first + j;
-        const float4 v0 = s.leaf_tris[3ULL * leaf];
-        const float4 v1 = s.leaf_tris[3ULL * leaf + 1];
-        const float4 v2 = s.leaf_tris[3ULL * leaf + 2];
-        TriangleHit th;
-        const int res =
-            triangle_test(v0, v1, v2, c.w.ro, c.w.rd, c.t_min, c.found ? c.best.t : c.t_max, false, th);
-        if (res == kTriFailure) {
-            c.w.failed = true;
-            continue;
-        }
-        if (res != kTriHit) {
-            continue;
-        }
-        const uint32_t prim = __float_as_uint(v0.w);
-        if (!c.found || precedes(th.t, c.w.inst, prim, c.best)) {
-            c.best.t = th.t;
-            c.best.instance = c.w.inst;
-            c.best.primitive = prim;
-            c.best.leaf = leaf;
-            c.found = true;
-        }
-    }
-    return true;
-}
-
-__device__ __forceinline__ ClosestResult closest_end(ClosestWalk& c) {
-    c.best.failed = c.w.failed;
-    if (!c.found) {
-        c.best.instance = 0xFFFFFFFFU;
-    }
-    return c.best;
-}
-
-// Closest hit of one ray (the standalone query kernel); k_trace runs the same steps with dynamic
-// ray fetch.
-template <bool SPH>
-__device__ ClosestResult closest_hit(const SceneView& s, F3 o, F3 d, float t_min, float t_max, uint32_t mask,
-                                     TraversalStack& stack) {
-    ClosestWalk c;
-    closest_begin(s, o, d, t_min, t_max, mask, stack, c);
-    while (closest_step<SPH>(s, stack, c)) {
-    }
-    return closest_end(c);
-}
-
-// Any hit in [t_min, t_max] (AccelBackend.cpp:114-147). One loop serves both levels, with one
-// visit for TLAS and BLAS nodes as in next_leaf; leaves go through the stack like nodes (the
-// nearest child on top), so every pass of the loop handles one entry per lane -- a node, an
-// instance range or one leaf -- and a lane stops at its first hit.
-// The set of leaves met does not depend on the order (the interval never shrinks), so neither does
-// the answer. Returns 1 occluded, 0 clear, -1 failure.
-template <bool SPH>
-__device__ int any_hit(const SceneView& s, F3 o, F3 d, float t_min, float t_max, uint32_t mask,
-                       TraversalStack& stack) {
-    bool failed = false;
-    const RayInv world = make_ray_inv(o, d);
-    int sp = 0;
-    push_instances(s, world, t_min, t_max, mask, stack, sp);
-    RayInv r = world;
-    F3 ro = o, rd = d;
-    while (sp > 0) {
-        const int entry = stack.get(--sp);
-        const uint32_t code = static_cast<uint32_t>(entry) ^ 0x80000000U;
-        const bool instance_level = entry < kLeafEntryMin;
-        if (instance_level && (code & kTlasFlag) == 0U) {
-            uint32_t inst = 0U;
-            enter_instance(s, code, world, o, d, t_min, t_max, mask, stack, sp, failed, inst, ro, rd, r);
-            continue;
-        }
-        if (!instance_level && entry < 0) {
-            const uint32_t packed = static_cast<uint32_t>(~entry);
-            const uint32_t first = packed >> kLeafCountBits;
-            const uint32_t n = (packed & (kMaxLeafSize - 1)) + 1U;
-            if (SPH && n == kSphereLeafCount) {
-                const int res = sphere_intersect(s.leaf_tris[3ULL * first], s.leaf_tris[3ULL * first + 1].x, ro, rd,
-                                                 t_min, t_max)
-                                    .outcome;
-                if (res == kSphereHit) {
-                    return 1;
-                }
-                failed = failed || res == kSphereFailure;
-                continue;
-            }
-            for (uint32_t j = 0; j < n; ++j) {
-                const uint32_t leaf = first + j;
-                TriangleHit th;
-                const int res = triangle_test(s.leaf_tris[3ULL * leaf], s.leaf_tris[3ULL * leaf + 1],
-                                              s.leaf_tris[3ULL * leaf + 2], ro, rd, t_min, t_max, false, th);
-                if (res == kTriHit) {
-                    return 1;
-                }
-                if (res == kTriFailure) {
-                    failed = true;
-                }
-            }
-            continue;
-        }
-        const int node = instance_level ? static_cast<int>(code & (kTlasFlag - 1U)) : entry;
-        int kids[4];
-        const int count = hit_children(instance_level ? world : r, s.nodes[node], t_min, t_max, kids);
-        push_children(kids, count, instance_level, stack, sp, failed);
-    }
-    return failed ? -1 : 0;
-}
 
 // Barycentrics of the winning triangle (correctly rounded e_i / det); for a sphere, its outward
 // object-space normal at the hit.
@@ -1047,7 +750,8 @@ cudaError_t launch_camera_rays(const PathSource& src, const bf200_sample_index_v
 
 __global__ void __launch_bounds__(256) k_regenerate(Wavefront w, PathSource src) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        w.counters[8] = 0ULL;  // k_trace's fetch cursor for this iteration
+        w.counters[kCounterTraceCursor] = 0ULL;
+        w.counters[kCounterOccludeCursor] = 0ULL;
     }
     const uint32_t stride = gridDim.x * blockDim.x;
     const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1079,108 +783,33 @@ __global__ void __launch_bounds__(256) k_regenerate(Wavefront w, PathSource src)
             const uint64_t id = base + rank;
             if (id < src.total) {
                 start_path(w, src, slot, id);
+                state = kSlotActive;
                 if ((w.status[slot] & 0xFFU) != 0U) {
                     w.state[slot] = kSlotDone;
+                    state = kSlotDone;
                 }
             }
+        }
+        // the slots to trace, one atomic per warp; every other slot is not routed this iteration
+        const bool active = in_range && state == kSlotActive;
+        const unsigned active_mask = __ballot_sync(0xFFFFFFFFU, active);
+        if (active_mask != 0U) {
+            const int leader = __ffs(active_mask) - 1;
+            unsigned long long at = 0;
+            if (static_cast<int>(threadIdx.x & 31U) == leader) {
+                at = atomicAdd(&w.counters[kCounterTraced], static_cast<unsigned long long>(__popc(active_mask)));
+            }
+            at = __shfl_sync(0xFFFFFFFFU, at, leader);
+            if (active) {
+                w.trace_queue[at + __popc(active_mask & ((1U << (threadIdx.x & 31U)) - 1U))] = slot;
+            }
+        }
+        if (in_range && !active) {
+            w.route[slot] = kRouteNone;
         }
     }
 }
 #endif  // BF200_KERNELS_MAIN_TU
-
-// ------------------------------------------------------------------------------------------------
-// k_trace: closest hit of every active slot's ray; writes the hit and the slot's shading route
-// ------------------------------------------------------------------------------------------------
-
-// Finishes one slot's trace: writes the hit (t and the barycentrics of the winning triangle) or
-// the miss or failure, and the slot's shading route.
-template <bool SPH>
-__device__ __forceinline__ void trace_finish(const SceneView& s, const Wavefront& w, uint32_t slot,
-                                             const ClosestResult& c, F3 o, F3 d, float t_min, float t_max) {
-    if (c.failed) {
-        w.status[slot] = (w.status[slot] & ~0xFFU) | kLaneTraversal;
-        w.state[slot] = kSlotDone;
-        w.route[slot] = kRouteNone;
-        return;
-    }
-    if (c.instance == 0xFFFFFFFFU) {
-        w.hit_id[slot] = make_uint2(0xFFFFFFFFU, 0U);
-        w.route[slot] = static_cast<uint8_t>(kRouteMiss);
-        return;
-    }
-    TriangleHit th;
-    if (!hit_barycentrics<SPH>(s, c, o, d, t_min, t_max, th)) {
-        w.status[slot] = (w.status[slot] & ~0xFFU) | kLaneNumerical;
-        w.state[slot] = kSlotDone;
-        w.route[slot] = kRouteNone;
-        return;
-    }
-    w.hit_tb[slot] = make_float4(c.t, th.b0, th.b1, th.b2);
-    // the winner's leaf record (its vertices, and the primitive index in the first record's w):
-    // shading reads the triangle from there, where this trace has just read it
-    w.hit_id[slot] = make_uint2(c.instance, c.leaf);
-    w.route[slot] = s.inst_route[c.instance];
-}
-
-// Persistent traversal with dynamic ray fetch: every lane keeps one ray in flight and, when its ray
-// is finished, takes the next slot from a cursor over [0, capacity) (one atomic per warp for all
-// of the warp's idle lanes), so a warp's lanes stay busy instead of waiting for its slowest ray.
-// Slots that are not active are marked unrouted as they are fetched.
-template <bool SPH>
-__global__ void __launch_bounds__(256, BF200_INTERSECT_MIN_BLOCKS) k_trace(SceneView s, Wavefront w) {
-    __shared__ int stack_columns[kSharedStackEntries * 256];
-    TraversalStack stack = thread_stack(stack_columns);
-    const uint32_t lane = threadIdx.x & 31U;
-    const uint32_t below = (1U << lane) - 1U;
-    uint32_t slot = 0xFFFFFFFFU;
-    bool drained = false;
-    ClosestWalk c;
-    while (true) {
-        const bool idle = slot == 0xFFFFFFFFU;
-        const unsigned idle_mask = __ballot_sync(0xFFFFFFFFU, idle);
-        if (idle_mask != 0U && !drained) {
-            unsigned long long base = 0;
-            if (lane == static_cast<uint32_t>(__ffs(idle_mask) - 1)) {
-                base = atomicAdd(&w.counters[8], static_cast<unsigned long long>(__popc(idle_mask)));
-            }
-            base = __shfl_sync(0xFFFFFFFFU, base, __ffs(idle_mask) - 1);
-            drained = base + __popc(idle_mask) >= w.capacity;
-            if (idle) {
-                const unsigned long long index = base + __popc(idle_mask & below);
-                if (index < w.capacity) {
-                    const uint32_t candidate = static_cast<uint32_t>(index);
-                    if (w.state[candidate] == kSlotActive) {
-                        slot = candidate;
-                        const float4 o4 = w.ray_o[slot], d4 = w.ray_d[slot];
-                        closest_begin(s, ld3(o4), ld3(d4), d4.w, o4.w, w.mask[slot], stack, c);
-                        w.status[slot] += 1U << 8;  // one extension segment
-                    } else {
-                        w.route[candidate] = kRouteNone;
-                    }
-                }
-            }
-        }
-        const bool busy = slot != 0xFFFFFFFFU;
-        const unsigned busy_mask = __ballot_sync(0xFFFFFFFFU, busy);
-        if (busy_mask == 0U) {
-            if (drained) {
-                break;
-            }
-            continue;
-        }
-        if (lane == static_cast<uint32_t>(__ffs(busy_mask) - 1) && idle_mask != 0U) {
-            // extension segments started in this pass (lanes that took an active slot)
-            const unsigned started = busy_mask & idle_mask;
-            if (started != 0U) {
-                atomicAdd(&w.counters[3], static_cast<unsigned long long>(__popc(started)));
-            }
-        }
-        if (busy && !closest_step<SPH>(s, stack, c)) {
-            trace_finish<SPH>(s, w, slot, closest_end(c), c.o, c.d, c.t_min, c.t_max);
-            slot = 0xFFFFFFFFU;
-        }
-    }
-}
 
 // ------------------------------------------------------------------------------------------------
 // Surface reconstruction (SceneSurfaceInteraction.cpp:54-350, 804-937)
@@ -2075,6 +1704,9 @@ __global__ void __launch_bounds__(256, BF200_SHADE_MIN_BLOCKS) k_shade(SceneView
     if constexpr (ADJ) {
         adjoint_zero(adjoint_sum);
     }
+    if (K == static_cast<int>(kClosureLambert) && blockIdx.x == 0 && threadIdx.x == 0) {
+        w.counters[kCounterTraced] = 0ULL;  // for the next iteration's k_regenerate
+    }
     const uint32_t begin = w.route_offsets[first_route], end = w.route_offsets[end_route];
     const uint32_t stride = gridDim.x * blockDim.x;
     uint32_t active_here = 0;
@@ -2490,57 +2122,6 @@ __global__ void __launch_bounds__(256, BF200_SHADE_MIN_BLOCKS) k_shade(SceneView
     }
 }
 
-// ------------------------------------------------------------------------------------------------
-// k_occlude: shadow rays of the compacted queue; unoccluded contributions join the path radiance
-// ------------------------------------------------------------------------------------------------
-
-template <bool ADJ, bool SPH>
-__global__ void __launch_bounds__(256, BF200_OCCLUDE_MIN_BLOCKS) k_occlude(SceneView s, Wavefront w, AdjointView a) {
-    __shared__ int stack_columns[kSharedStackEntries * 256];
-    __shared__ double adjoint_sum[ADJ ? kAdjointWords : 1];
-    if constexpr (ADJ) {
-        adjoint_zero(adjoint_sum);
-    }
-    TraversalStack stack = thread_stack(stack_columns);
-    const uint32_t count = w.shadow_offsets[1];
-    const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += stride) {
-        const uint32_t slot = w.shadow_queue[i];
-        const float4 o = w.shadow_o[slot], d = w.shadow_d[slot];
-        const int occluded = any_hit<SPH>(s, ld3(o), ld3(d), 0.0F, o.w, w.mask[slot], stack);
-        if (occluded < 0) {
-            w.status[slot] = (w.status[slot] & ~0xFFU) | kLaneTraversal;
-            w.state[slot] = kSlotDone;
-            continue;
-        }
-        if (occluded == 0) {
-            const float4 c = w.shadow_c[slot];
-            float4 r = w.radiance[slot];
-            r.x = r.x + c.x;
-            r.y = r.y + c.y;
-            r.z = r.z + c.z;
-            r.w = r.w + c.w;
-            w.radiance[slot] = r;
-            if constexpr (ADJ) {
-                const AdjointLane al = adjoint_lane(a, w.path_id[slot]);
-                if (al.on) {  // the light's radiance scales this contribution; so may the roughness
-                    const float added[4] = {c.x, c.y, c.z, c.w};
-                    const double e = adjoint_dot(al, added);
-                    atomicAdd(&adjoint_sum[kAdjointEmission], e);
-                    const uint4 score = a.shadow_score[slot];
-                    if (score.w != 0U) {
-                        atomicAdd(&adjoint_sum[score.z * kAdjointStride + 4U], e * __uint_as_float(score.x));
-                        atomicAdd(&adjoint_sum[score.z * kAdjointStride + 5U], e * __uint_as_float(score.y));
-                    }
-                }
-            }
-        }
-    }
-    if constexpr (ADJ) {
-        adjoint_flush(adjoint_sum, a.gradients);
-    }
-}
-
 #ifdef BF200_KERNELS_MAIN_TU
 // ------------------------------------------------------------------------------------------------
 // k_film: CIE 1931 XYZ -> linear sRGB -> add_sample(x, y, rgb, 1) in sample order per pixel
@@ -2679,55 +2260,6 @@ __global__ void __launch_bounds__(256) k_adjoint_image(const float4* film32, con
 }
 #endif  // BF200_KERNELS_MAIN_TU
 
-// Standalone closest-hit / occlusion queries (ClosestHit.hpp:21-28, Occlusion.hpp:19-26).
-template <bool SPH>
-__global__ void __launch_bounds__(128) k_query_closest(SceneView s, const bf200_ray_v1* rays, uint64_t n,
-                                                      bf200_hit_v1* hits) {
-    __shared__ int stack_columns[kSharedStackEntries * 128];
-    TraversalStack stack = thread_stack(stack_columns);
-    for (uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < n;
-         i += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
-        const bf200_ray_v1 r = rays[i];
-        const F3 o{r.origin[0], r.origin[1], r.origin[2]}, d{r.direction[0], r.direction[1], r.direction[2]};
-        const ClosestResult c = closest_hit<SPH>(s, o, d, r.t_min, r.t_max, r.mask, stack);
-        bf200_hit_v1 h;
-        h.t = 0.0F;
-        h.barycentrics[0] = h.barycentrics[1] = h.barycentrics[2] = 0.0F;
-        h.instance_index = 0xFFFFFFFFU;
-        h.primitive_index = 0xFFFFFFFFU;
-        h.status = c.failed ? kLaneTraversal : 0U;
-        h.reserved = 0U;
-        if (!c.failed && c.instance != 0xFFFFFFFFU) {
-            TriangleHit th;
-            if (hit_barycentrics<SPH>(s, c, o, d, r.t_min, r.t_max, th)) {
-                h.t = c.t;
-                h.barycentrics[0] = th.b0;
-                h.barycentrics[1] = th.b1;
-                h.barycentrics[2] = th.b2;
-                h.instance_index = c.instance;
-                h.primitive_index = c.primitive;
-            } else {
-                h.status = kLaneNumerical;
-            }
-        }
-        hits[i] = h;
-    }
-}
-
-template <bool SPH>
-__global__ void __launch_bounds__(128) k_query_occlusion(SceneView s, const bf200_ray_v1* rays, uint64_t n,
-                                                        uint32_t* out) {
-    __shared__ int stack_columns[kSharedStackEntries * 128];
-    TraversalStack stack = thread_stack(stack_columns);
-    for (uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < n;
-         i += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
-        const bf200_ray_v1 r = rays[i];
-        const F3 o{r.origin[0], r.origin[1], r.origin[2]}, d{r.direction[0], r.direction[1], r.direction[2]};
-        const int occ = any_hit<SPH>(s, o, d, r.t_min, r.t_max, r.mask, stack);
-        out[i] = occ < 0 ? 2U : static_cast<uint32_t>(occ);
-    }
-}
-
 // The shading kernels of one wavefront iteration: the Lambert route's, and the others.
 template <bool ADJ, bool CONE, bool TREE>
 void launch_shade_lambert(const SceneView& s, const Wavefront& w, const PathSource& src, const TransportParams& p,
@@ -2747,6 +2279,12 @@ void launch_shade_others(const SceneView& s, const Wavefront& w, const PathSourc
 }
 
 #ifdef BF200_KERNELS_MAIN_TU
+}  // namespace bf200
+
+#include "bf200_pool.cuh"
+
+namespace bf200 {
+
 // The shading launchers are instantiated in their own translation units (bf200_shade_*.cu), which
 // compile in parallel.
 #define BF200_SHADE_LAUNCHERS(ADJ, CONE, TREE)                                                                    \
@@ -2821,13 +2359,19 @@ cudaError_t launch_stage(int stage, const SceneView& s, const Wavefront& w, cons
         return cudaGetLastError();
     }
     if (stage == 1) {
+        *launches += 2U;
         if (s.sphere_count != 0U) {
-            k_trace<true><<<grid, 256, 0, stream>>>(s, w);
+            e = launch_pool(k_trace<true>, w.capacity, stream, s, w);
+            if (e == cudaSuccess) {
+                k_hits<true><<<grid, 256, 0, stream>>>(s, w);
+            }
         } else {
-            k_trace<false><<<grid, 256, 0, stream>>>(s, w);
+            e = launch_pool(k_trace<false>, w.capacity, stream, s, w);
+            if (e == cudaSuccess) {
+                k_hits<false><<<grid, 256, 0, stream>>>(s, w);
+            }
         }
-        *launches += 1U;
-        return cudaGetLastError();
+        return e == cudaSuccess ? cudaGetLastError() : e;
     }
     if (stage == 2) {
         // route the traced slots, shade each route with its own kernel, then queue the shadow rays
@@ -2857,19 +2401,13 @@ cudaError_t launch_stage(int stage, const SceneView& s, const Wavefront& w, cons
                                  w.counters + 0, nullptr, stream, launches);
     }
     const AdjointView a = adjoint != nullptr ? *adjoint : AdjointView{};
-    if (s.sphere_count != 0U) {
-        if (adjoint != nullptr) {
-            k_occlude<true, true><<<grid, 256, 0, stream>>>(s, w, a);
-        } else {
-            k_occlude<false, true><<<grid, 256, 0, stream>>>(s, w, a);
-        }
-    } else if (adjoint != nullptr) {
-        k_occlude<true, false><<<grid, 256, 0, stream>>>(s, w, a);
-    } else {
-        k_occlude<false, false><<<grid, 256, 0, stream>>>(s, w, a);
-    }
     *launches += 1U;
-    return cudaGetLastError();
+    if (s.sphere_count != 0U) {
+        return adjoint != nullptr ? launch_pool(k_occlude<true, true>, w.capacity, stream, s, w, a)
+                                  : launch_pool(k_occlude<false, true>, w.capacity, stream, s, w, a);
+    }
+    return adjoint != nullptr ? launch_pool(k_occlude<true, false>, w.capacity, stream, s, w, a)
+                              : launch_pool(k_occlude<false, false>, w.capacity, stream, s, w, a);
 }
 
 cudaError_t launch_retire(const Wavefront& w, const PathSource& src, uint32_t grid, cudaStream_t stream) {
@@ -2903,22 +2441,22 @@ cudaError_t launch_adjoint_image(const float4* film32, const double* film64, con
 
 cudaError_t launch_queries(const SceneView& s, const bf200_ray_v1* rays, uint64_t n, bf200_hit_v1* hits,
                            uint32_t* occluded, cudaStream_t stream) {
-    const uint64_t blocks64 = (n + 127U) / 128U;
-    const uint32_t blocks = static_cast<uint32_t>(blocks64 < 65535U ? (blocks64 == 0 ? 1 : blocks64) : 65535U);
     if (hits != nullptr) {
-        if (s.sphere_count != 0U) {
-            k_query_closest<true><<<blocks, 128, 0, stream>>>(s, rays, n, hits);
-        } else {
-            k_query_closest<false><<<blocks, 128, 0, stream>>>(s, rays, n, hits);
+        cudaError_t e = s.sphere_count != 0U ? launch_pool(k_query_closest<true>, n, stream, s, rays, n, hits)
+                                             : launch_pool(k_query_closest<false>, n, stream, s, rays, n, hits);
+        if (e == cudaSuccess) {
+            const uint32_t blocks = static_cast<uint32_t>(std::min<uint64_t>((n + 127U) / 128U, 65535U));
+            if (s.sphere_count != 0U) {
+                k_query_hits<true><<<blocks, 128, 0, stream>>>(s, rays, n, hits);
+            } else {
+                k_query_hits<false><<<blocks, 128, 0, stream>>>(s, rays, n, hits);
+            }
+            e = cudaGetLastError();
         }
-    } else {
-        if (s.sphere_count != 0U) {
-            k_query_occlusion<true><<<blocks, 128, 0, stream>>>(s, rays, n, occluded);
-        } else {
-            k_query_occlusion<false><<<blocks, 128, 0, stream>>>(s, rays, n, occluded);
-        }
+        return e;
     }
-    return cudaGetLastError();
+    return s.sphere_count != 0U ? launch_pool(k_query_occlusion<true>, n, stream, s, rays, n, occluded)
+                                : launch_pool(k_query_occlusion<false>, n, stream, s, rays, n, occluded);
 }
 
 #endif  // BF200_KERNELS_MAIN_TU
