@@ -852,7 +852,7 @@ static __device__ bool transform_position_with_error(const SceneView& s, uint32_
         }
         err[row] = __double2float_rn(bound);
         if (static_cast<double>(err[row]) < bound) {
-            err[row] = nextafterf(err[row], kInf);
+            err[row] = next_float(err[row], true);
         }
     }
     out.position = world;
@@ -1069,7 +1069,7 @@ static __device__ void sample_mesh_light(const SceneView& s, const LightInfo& li
         point[axis] = fmaf(bary[0], cs[0][axis], fmaf(bary[1], cs[1][axis], q2));
         const float magnitude = fabsf(q0) + fabsf(q1) + fabsf(q2);
         const float arithmetic = fmaf(gamma12, magnitude, underflow);
-        error[axis] = nextafterf(base[axis] + arithmetic, kInf);
+        error[axis] = next_float(base[axis] + arithmetic, true);
     }
     out.position = F3{point[0], point[1], point[2]};
     out.error = F3{error[0], error[1], error[2]};
@@ -1131,6 +1131,21 @@ __device__ __forceinline__ float scale_radiometric(float value, const float* num
     }
     if (value == 0.0F) {
         return 0.0F;
+    }
+    {
+        float direct = value, least = value;
+        for (int i = 0; i < n; ++i) {
+            direct *= num[i];
+            least = fminf(least, fminf(num[i], direct));
+        }
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            direct /= den[i];
+            least = fminf(least, fminf(den[i], direct));
+        }
+        if (least >= kMinNormal && direct <= kMaxFloat) {
+            return direct;
+        }
     }
     int exponent = 0;
     float fraction = frexpf(value, &exponent);
@@ -1260,7 +1275,7 @@ __device__ __forceinline__ F3 contract_point_endpoint(F3 point, F3 error, F3 to_
         if (!isfinite(candidate) || candidate < contraction) {
             lane.fail();
         }
-        contraction = (d[a] != 0.0F && e[a] != 0.0F) ? nextafterf(candidate, kInf) : candidate;
+        contraction = (d[a] != 0.0F && e[a] != 0.0F) ? next_float(candidate, true) : candidate;
     }
     if (!isfinite(contraction)) {
         lane.fail();
@@ -1273,7 +1288,7 @@ __device__ __forceinline__ F3 contract_point_endpoint(F3 point, F3 error, F3 to_
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         if (d[a] != 0.0F) {
-            c[a] = nextafterf(c[a], d[a] > 0.0F ? -kInf : kInf);
+            c[a] = next_float(c[a], !(d[a] > 0.0F));
         }
     }
     const F3 out{c[0], c[1], c[2]};
@@ -1403,6 +1418,13 @@ __device__ __forceinline__ void add_weighted_emission(float4& acc, const float4 
         if (bv[l] == 0.0F || le[l] == 0.0F || wgt == 0.0F) {
             continue;
         }
+        const float num[3] = {bv[l], le[l], wgt};
+        const float den[1] = {1.0F};
+        float direct;
+        if (Factors<3, 1>(num, den).direct(direct)) {
+            r[l] = r[l] + direct;
+            continue;
+        }
         int e1 = 0, e2 = 0, e3 = 0, en = 0;
         const float significand = frexpf(bv[l], &e1) * frexpf(le[l], &e2) * frexpf(wgt, &e3);
         const float normalized = frexpf(significand, &en);
@@ -1515,7 +1537,7 @@ __device__ void direct_lighting(const SceneView& s, const TransportParams& p, co
         }
         float length = 1.0F;
         unit_segment(origin, endpoint, ls.direction, sd, length, lane);
-        t_max = nextafterf(length, 0.0F);
+        t_max = next_float(length, false);
         if (!(t_max > 0.0F) || !isfinite(t_max)) {
             lane.fail();
         }
@@ -1962,6 +1984,10 @@ __global__ void __launch_bounds__(256, BF200_SHADE_MIN_BLOCKS) k_shade(SceneView
 #pragma unroll
                                 for (int l = 0; l < 4; ++l) {
                                     const float num[4] = {bv[l], bs.value[l], cosine, 1.0F};
+                                    const float den[1] = {bs.pdf};
+                                    if (Factors<4, 1>(num, den).direct(nb[l])) {
+                                        continue;
+                                    }
                                     float significand = 1.0F;
                                     int exponent = 0;
                                     bool zero = false;
@@ -2136,6 +2162,11 @@ struct SensorView {
 __device__ __forceinline__ float sensor_term(float c, float r, float n, float p) {
     if (c == 0.0F || r == 0.0F) {
         return 0.0F;
+    }
+    const float num[3] = {c, r, n}, den[1] = {p};
+    float direct;
+    if (Factors<3, 1>(num, den).direct(direct)) {
+        return direct;
     }
     int ec = 0, er = 0, en = 0, ep = 0;
     const float mc = frexpf(c, &ec), mr = frexpf(r, &er), mn = frexpf(n, &en), mp = frexpf(p, &ep);
