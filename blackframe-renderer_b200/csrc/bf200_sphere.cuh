@@ -188,9 +188,13 @@ __device__ __forceinline__ float fused_dot3(F3 a, F3 b) { return fmaf(a.x, b.x, 
 
 // ------------------------------------------------------------------------------------------------
 // Fast path for the two expansion values. Two facts make it exact:
-// * With every scaled input component 0 or of magnitude >= 2^-8 (least significant bit
-//   >= 2^-31), every nonzero product and product error the expansions form is a multiple of at
-//   least 2^-124, so none is subnormal and the reference's representability checks all pass.
+// * A float of magnitude >= 2^e is a multiple of 2^(e - 23). The constant's terms multiply two
+//   components of (rel, r), the discriminant's two of (rel, r) with two of d. So when the smallest
+//   nonzero magnitudes of the two groups multiply to at least 2^-15 (their exponents then add to at
+//   least -17), every nonzero product and product error the expansions form is a multiple of at least
+//   2^(-2 * 17 - 92) = 2^-126, none is subnormal, and the reference's representability checks all
+//   pass. (Every component of one group at least 2^-8 had been asked for, which 2 to 3 % of the rays
+//   of a Cornell box miss: a warp then waits for one lane's expansions on every third test.)
 // * Summing a nonoverlapping expansion from its smallest component up, as the reference does,
 //   lands within about 2 u_f ulp of its exact value X (u_f = 2^-24). So when X lies farther than
 //   2^-12 ulp from every float rounding boundary, that sum is the float nearest to X.
@@ -225,7 +229,13 @@ __device__ __forceinline__ DoubleDouble dd_scale(DoubleDouble x, double y) {
     return dd_two_sum(p, e);
 }
 
-__device__ __forceinline__ bool coarse_component(float x) { return x == 0.0F || fabsf(x) >= 0.00390625F; }
+// The smallest nonzero magnitude of a group of scaled components (1 when there is none).
+__device__ __forceinline__ float least_magnitude(float x, float y, float z) {
+    float least = 1.0F;
+    least = x != 0.0F ? fminf(least, fabsf(x)) : least;
+    least = y != 0.0F ? fminf(least, fabsf(y)) : least;
+    return z != 0.0F ? fminf(least, fabsf(z)) : least;
+}
 
 // The float nearest to X = x.hi + x.lo (known to within err) when X is certainly farther than
 // 2^-12 ulp from each rounding boundary of that float; false otherwise.
@@ -249,8 +259,8 @@ __device__ __forceinline__ bool certified_nearest(DoubleDouble x, double err, fl
 // c = |rel|^2 - r^2 and the discriminant |d|^2 r^2 - |rel x d|^2 of the scaled inputs by the fast
 // path; false when the fast path is not certain (the expansions then decide).
 __device__ __forceinline__ bool sphere_values_fast(F3 srel, F3 sd, float sr, float& c, int& disc_sign, float& disc) {
-    if (!coarse_component(srel.x) || !coarse_component(srel.y) || !coarse_component(srel.z) ||
-        !coarse_component(sd.x) || !coarse_component(sd.y) || !coarse_component(sd.z) || !coarse_component(sr)) {
+    const float least_spatial = fminf(least_magnitude(srel.x, srel.y, srel.z), fabsf(sr));
+    if (!(least_spatial * least_magnitude(sd.x, sd.y, sd.z) >= 0x1p-15F)) {
         return false;
     }
     const double rx = srel.x, ry = srel.y, rz = srel.z, dx = sd.x, dy = sd.y, dz = sd.z, r2 = double(sr) * sr;

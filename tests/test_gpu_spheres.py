@@ -153,3 +153,42 @@ def test_sphere_scene_checks(ctx):
     with pytest.raises(runtime.Bf200Error) as info:
         ctx.create_scene(bad)
     assert info.value.status == 1  # INVALID_ARGUMENT, as SphereT::create
+
+
+@pytest.mark.parametrize("spatial,directional", [(0, 0), (8, 6), (9, 6), (14, 0), (12, 3), (15, 1), (4, 11), (0, 15),
+                                                 (10, 8), (16, 0), (0, 16)])
+def test_small_components_match_the_oracle(ctx, spatial, directional):
+    """Rays with one component of the centre offset and one of the direction tiny, on both sides of the
+    rule that lets the double-double evaluation stand for the expansions (smallest magnitudes of the
+    two groups multiplying to 2^-15)."""
+    rng = np.random.default_rng(100 * spatial + directional)
+    n = 600
+    radius, centre = np.float32(0.75), np.array([0.25, -0.5, 1.0], np.float32)
+    offset = rng.normal(size=(n, 3))
+    offset *= (rng.uniform(0.2, 3.0, n) / np.linalg.norm(offset, axis=1))[:, None]  # inside and outside
+    target = rng.normal(size=(n, 3))
+    target *= (rng.uniform(0.0, 0.8, n) / np.linalg.norm(target, axis=1))[:, None]
+    direction = target - offset
+    direction /= np.linalg.norm(direction, axis=1, keepdims=True)
+    axis, other = rng.integers(0, 3, n), rng.integers(0, 3, n)
+    rows = np.arange(n)
+    if spatial:
+        offset[rows, axis] = np.copysign(2.0 ** -spatial * rng.uniform(1.0, 2.0, n), offset[rows, axis])
+    if directional:
+        direction[rows, other] = np.copysign(2.0 ** -directional * rng.uniform(1.0, 2.0, n), direction[rows, other])
+    origin = (centre + offset).astype(np.float32)
+    rays = rays_from(np.concatenate([origin, direction.astype(np.float32), np.zeros((n, 1)),
+                                     np.full((n, 1), np.inf)], axis=1))
+    builder = sphere_scene([(*centre, radius)])
+    oracle = Oracle(device_trig=True)
+    handle = oracle.scene(builder)
+    expected = oracle.closest_hits(handle, rays)
+    oracle.destroy(handle)
+    scene = ctx.create_scene(builder)
+    got = ctx.closest_hits(scene, rays)
+    scene.close()
+    want = np.frombuffer(expected, np.uint32).reshape(n, 8)
+    have = np.frombuffer(got, np.uint32).reshape(n, 8)
+    kept = want[:, 6] == 0  # the reference's test may report a product it cannot represent
+    assert kept.mean() > 0.9 and (want[kept, 4] == 0).mean() > 0.2
+    assert np.array_equal(have[kept], want[kept])
