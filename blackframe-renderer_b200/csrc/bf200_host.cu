@@ -55,7 +55,7 @@ struct bf200_context {
     size_t film_radiance_bytes = 0;
     void* film_staging = nullptr;   // device copy of a host film
     size_t film_staging_bytes = 0;
-    void* batch_staging = nullptr;  // device copies of host path inputs and results
+    void* batch_staging = nullptr;  // device copies of host path inputs and results, and of query rays and answers
     size_t batch_staging_bytes = 0;
     // film batches (bf200_render_films_device): one stream, event, arena slice, pinned counter
     // block and radiance buffer per lane, kept across calls
@@ -3386,16 +3386,18 @@ static blackframe_status run_queries(bf200_context* c, const bf200_scene* s, con
         return BLACKFRAME_STATUS_SUCCESS;
     }
     cudaSetDevice(c->device);
-    bf200_ray_v1* d_rays = nullptr;
-    void* d_out = nullptr;
+    // device copies of the rays and the answers in the context's batch staging: with an allocation and
+    // a release of each per call, 20,001 rays took 1.0 ms, and 0.29 ms without
     const size_t out_bytes = n * (hits != nullptr ? sizeof(bf200_hit_v1) : sizeof(uint32_t));
-    cudaError_t e = cudaMalloc(&d_rays, n * sizeof(bf200_ray_v1));
-    if (e == cudaSuccess) {
-        e = cudaMalloc(&d_out, out_bytes);
+    const size_t ray_bytes = (n * sizeof(bf200_ray_v1) + 255) & ~size_t(255);
+    if (const auto st = grow_workspace(c, &c->batch_staging, &c->batch_staging_bytes, ray_bytes + out_bytes,
+                                       "query staging");
+        st != BLACKFRAME_STATUS_SUCCESS) {
+        return st;
     }
-    if (e == cudaSuccess) {
-        e = cudaMemcpyAsync(d_rays, rays, n * sizeof(bf200_ray_v1), cudaMemcpyHostToDevice, c->stream);
-    }
+    auto* d_rays = static_cast<bf200_ray_v1*>(c->batch_staging);
+    void* d_out = static_cast<char*>(c->batch_staging) + ray_bytes;
+    cudaError_t e = cudaMemcpyAsync(d_rays, rays, n * sizeof(bf200_ray_v1), cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess) {
         e = launch_queries(s->view, d_rays, n, hits != nullptr ? static_cast<bf200_hit_v1*>(d_out) : nullptr,
                            hits != nullptr ? nullptr : static_cast<uint32_t*>(d_out), c->stream);
@@ -3404,11 +3406,8 @@ static blackframe_status run_queries(bf200_context* c, const bf200_scene* s, con
         e = cudaMemcpyAsync(hits != nullptr ? static_cast<void*>(hits) : static_cast<void*>(occluded), d_out, out_bytes,
                             cudaMemcpyDeviceToHost, c->stream);
     }
-    if (e == cudaSuccess) {
-        e = cudaStreamSynchronize(c->stream);
-    }
-    cudaFree(d_rays);
-    cudaFree(d_out);
+    const cudaError_t done = cudaStreamSynchronize(c->stream);
+    e = e == cudaSuccess ? done : e;
     return e == cudaSuccess ? BLACKFRAME_STATUS_SUCCESS : cuda_fail(c, e, "query");
 }
 
