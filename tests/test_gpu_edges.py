@@ -80,3 +80,36 @@ def test_edge_and_vertex_rays_bit_exact():
                 f"{(occluded != found).sum()} occlusion answers differ from the closest hits"
         scene.close()
     oracle.destroy(handle)
+
+
+@pytest.mark.parametrize("distance", [1.0, 100.0, 10000.0])
+@pytest.mark.parametrize("exponent", [4, 10, 16, 22])
+def test_small_barycentrics_bit_exact(exponent, distance):
+    """Hits whose smallest barycentric weights are about 2^-exponent, seen from near and far: t and the
+    weights equal the exact ones whichever evaluation certifies them."""
+    builder, mesh = edge_scene()
+    rng = np.random.default_rng(exponent)
+    n = 1500
+    p = mesh.positions.astype(np.float32)
+    tri = mesh.triangles[rng.integers(0, len(mesh.triangles), n)]
+    small = 2.0 ** -exponent * rng.uniform(0.5, 2.0, (n, 2))
+    small[:, 1] = np.where(rng.random(n) < 0.5, small[:, 1], rng.uniform(0.1, 0.5, n))  # near a corner or an edge
+    weights = np.concatenate([small, 1.0 - small.sum(axis=1, keepdims=True)], axis=1)
+    weights = rng.permuted(weights, axis=1)
+    target = sum(weights[:, k:k + 1] * p[tri[:, k]] for k in range(3))
+    direction = rng.normal(size=(n, 3))
+    direction /= np.linalg.norm(direction, axis=1, keepdims=True)
+    direction = direction.astype(np.float32)
+    origin = (target - distance * direction).astype(np.float32)
+    rays = ray_array(origin, direction, np.full(n, np.inf, np.float32))
+    oracle = Oracle(device_trig=True)
+    handle = oracle.scene(builder)
+    expected = oracle.closest_hits(handle, rays)
+    oracle.destroy(handle)
+    with runtime.Context(0, path_capacity=1 << 12) as ctx:
+        scene = ctx.create_scene(builder)
+        got = ctx.closest_hits(scene, rays)
+        scene.close()
+    want = np.frombuffer(expected, np.uint32).reshape(n, 8)
+    assert (want[:, 6] == 0).all() and (want[:, 4] != 0xFFFFFFFF).mean() > 0.5
+    assert np.array_equal(np.frombuffer(got, np.uint32).reshape(n, 8), want)
