@@ -99,3 +99,24 @@ def test_next_float_steps():
         with np.errstate(all="ignore"):
             expected = np.nextafter(v, F(np.inf) if up else F(-np.inf))
         assert np.array_equal(stepped.view(np.uint32), expected.view(np.uint32))
+
+
+def test_unit_normals_by_one_reciprocal_root():
+    """transform_normal's rule: where the float around a reciprocal-root normal is certain (2^-46), the
+    divided and scaled form rounds to it too."""
+    rng = np.random.default_rng(9)
+    v = rng.normal(size=(400_000, 3)) * np.exp2(rng.uniform(-60.0, 60.0, (400_000, 1)))
+    v[::5, 0] *= np.exp2(rng.uniform(-40.0, 0.0, len(v[::5])))
+    v[::7, 1] = 0.0
+    squared = v[:, 0] * v[:, 0] + (v[:, 1] * v[:, 1] + v[:, 2] * v[:, 2])
+    root = 1.0 / np.sqrt(squared)
+    root = root * (1.0 + rng.choice([-2.0, 0.0, 2.0], len(v)) * 2.0 ** -52)  # a root some ulps off
+    q = v * root[:, None]
+    slack = np.abs(q) * 2.0 ** -46
+    low, high = (q - slack).astype(F), (q + slack).astype(F)
+    certain = (low == high).all(axis=1)
+    scaled = v / np.abs(v).max(axis=1, keepdims=True)
+    length = np.sqrt(scaled[:, 0] * scaled[:, 0] + (scaled[:, 1] * scaled[:, 1] + scaled[:, 2] * scaled[:, 2]))
+    expected = (scaled / length[:, None]).astype(F)
+    assert certain.mean() > 0.999
+    assert np.array_equal(low[certain].view(np.uint32), expected[certain].view(np.uint32))
