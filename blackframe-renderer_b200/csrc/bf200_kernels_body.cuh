@@ -2444,12 +2444,12 @@ cudaError_t launch_stage(int stage, const SceneView& s, const Wavefront& w, cons
     if (stage == 1) {
         *launches += 2U;
         if (s.sphere_count != 0U) {
-            e = launch_pool(k_trace<true>, w.capacity, stream, s, w);
+            e = launch_pool<false>(k_trace<true>, w.capacity, stream, s, w);
             if (e == cudaSuccess) {
                 k_hits<true><<<grid, 256, 0, stream>>>(s, w);
             }
         } else {
-            e = launch_pool(k_trace<false>, w.capacity, stream, s, w);
+            e = launch_pool<false>(k_trace<false>, w.capacity, stream, s, w);
             if (e == cudaSuccess) {
                 k_hits<false><<<grid, 256, 0, stream>>>(s, w);
             }
@@ -2486,11 +2486,11 @@ cudaError_t launch_stage(int stage, const SceneView& s, const Wavefront& w, cons
     const AdjointView a = adjoint != nullptr ? *adjoint : AdjointView{};
     *launches += 1U;
     if (s.sphere_count != 0U) {
-        return adjoint != nullptr ? launch_pool(k_occlude<true, true>, w.capacity, stream, s, w, a)
-                                  : launch_pool(k_occlude<false, true>, w.capacity, stream, s, w, a);
+        return adjoint != nullptr ? launch_pool<true>(k_occlude<true, true>, w.capacity, stream, s, w, a)
+                                  : launch_pool<true>(k_occlude<false, true>, w.capacity, stream, s, w, a);
     }
-    return adjoint != nullptr ? launch_pool(k_occlude<true, false>, w.capacity, stream, s, w, a)
-                              : launch_pool(k_occlude<false, false>, w.capacity, stream, s, w, a);
+    return adjoint != nullptr ? launch_pool<true>(k_occlude<true, false>, w.capacity, stream, s, w, a)
+                              : launch_pool<true>(k_occlude<false, false>, w.capacity, stream, s, w, a);
 }
 
 cudaError_t launch_retire(const Wavefront& w, const PathSource& src, uint32_t grid, cudaStream_t stream) {
@@ -2525,8 +2525,8 @@ cudaError_t launch_adjoint_image(const float4* film32, const double* film64, con
 cudaError_t launch_queries(const SceneView& s, const bf200_ray_v1* rays, uint64_t n, bf200_hit_v1* hits,
                            uint32_t* occluded, cudaStream_t stream) {
     if (hits != nullptr) {
-        cudaError_t e = s.sphere_count != 0U ? launch_pool(k_query_closest<true>, n, stream, s, rays, n, hits)
-                                             : launch_pool(k_query_closest<false>, n, stream, s, rays, n, hits);
+        cudaError_t e = s.sphere_count != 0U ? launch_pool<false>(k_query_closest<true>, n, stream, s, rays, n, hits)
+                                             : launch_pool<false>(k_query_closest<false>, n, stream, s, rays, n, hits);
         if (e == cudaSuccess) {
             const uint32_t blocks = static_cast<uint32_t>(std::min<uint64_t>((n + 127U) / 128U, 65535U));
             if (s.sphere_count != 0U) {
@@ -2538,8 +2538,8 @@ cudaError_t launch_queries(const SceneView& s, const bf200_ray_v1* rays, uint64_
         }
         return e;
     }
-    return s.sphere_count != 0U ? launch_pool(k_query_occlusion<true>, n, stream, s, rays, n, occluded)
-                                : launch_pool(k_query_occlusion<false>, n, stream, s, rays, n, occluded);
+    return s.sphere_count != 0U ? launch_pool<true>(k_query_occlusion<true>, n, stream, s, rays, n, occluded)
+                                : launch_pool<true>(k_query_occlusion<false>, n, stream, s, rays, n, occluded);
 }
 
 #endif  // BF200_KERNELS_MAIN_TU

@@ -15,8 +15,13 @@ namespace bf200 {
 
 // Rays per lane, threads per block, resident blocks per SM (the registers a walk needs allow four).
 // Measured on the BVH-stress frame (16 samples; trace + occlude): 1 ray 174 ms (6 blocks), 2 rays 130
-// ms, 3 rays 126 ms; 5 and 6 blocks with 2 rays 154 and 188 ms, from spills and the smaller L1.
-constexpr int kPoolRays = 3, kPoolThreads = 128, kPoolBlocks = 4;
+// ms, 3 rays 126 ms; 5 and 6 blocks with 2 rays 154 and 188 ms, from spills and the smaller L1. Shadow
+// rays deal their leaves' triangles over the warp (2 rays suffice then: occlude 34.6 -> 32.7 ms, Cornell
+// box with spheres 13.4 -> 12.8 ms). Closest hits do not: 89.7 -> 87.1 ms there, but 30.8 -> 32.5 ms in
+// the box, whose leaves hold one or two triangles.
+constexpr int kPoolThreads = 128, kPoolBlocks = 4;
+template <bool ANY>
+constexpr int kPoolRays = ANY ? 2 : 3;
 // Stack entries of a ray in shared memory; deeper ones, which few walks reach, are local.
 constexpr int kPoolStack = 15;
 // A node visit is repeated in registers while at least this many sixteenths of the lanes that began
@@ -40,7 +45,16 @@ enum PoolWord : int {
 constexpr int kPoolWords = kPoolFrames + kPoolStack;
 constexpr uint32_t kPoolSpMask = 0xFFU, kPoolAxes = 0x700U, kPoolFound = 0x800U, kPoolFailed = 0x1000U;
 constexpr int kPoolAxesShift = 8;
-constexpr size_t kPoolSharedBytes = sizeof(uint32_t) * kPoolWords * kPoolRays * kPoolThreads;
+// One operation's leaf triangles, per warp: the tests of all its lanes (at most 4 each), and the lane and
+// ray that asked for each.
+constexpr uint32_t kPoolTests = 128U;
+template <bool ANY>
+constexpr int kPoolRayWords = kPoolWords * kPoolRays<ANY> * kPoolThreads;
+template <bool ANY>
+constexpr size_t kPoolSharedBytes =
+    sizeof(uint32_t) * kPoolRayWords<ANY> +
+    (ANY ? (sizeof(uint32_t) + sizeof(uint8_t)) * kPoolTests * (kPoolThreads / 32) : 0U);
+constexpr uint32_t kPoolMiss = 0xFFFFFFFFU, kPoolFailure = 0xFFFFFFFEU;  // a test's answer
 
 // The entry of a ray whose walk has ended (no stack code).
 constexpr int kPoolDone = INT_MAX;
@@ -111,12 +125,13 @@ __device__ __forceinline__ uint32_t pool_op(int entry, bool world) {
 template <bool ANY, bool SPH, class Job>
 __device__ __forceinline__ void pool_walk(const SceneView& s, Job& job, uint32_t* shared) {
     uint32_t* const column = shared + threadIdx.x;
-    int deep[kPoolRays][kTraversalStack - kPoolStack];
-    int entry[kPoolRays];  // each ray's next entry, popped
-    uint32_t due_op[kPoolRays];
+    constexpr int kRays = kPoolRays<ANY>;
+    int deep[kRays][kTraversalStack - kPoolStack];
+    int entry[kRays];  // each ray's next entry, popped
+    uint32_t due_op[kRays];
     uint32_t world = 0U;  // bit k: ray k is in the world's frame
 #pragma unroll
-    for (int k = 0; k < kPoolRays; ++k) {
+    for (int k = 0; k < kRays; ++k) {
         entry[k] = kPoolDone;
         due_op[k] = kPoolFetch;
     }
@@ -124,7 +139,7 @@ __device__ __forceinline__ void pool_walk(const SceneView& s, Job& job, uint32_t
         // the operation most lanes can run
         uint32_t mine = 0U;
 #pragma unroll
-        for (int k = 0; k < kPoolRays; ++k) {
+        for (int k = 0; k < kRays; ++k) {
             mine |= 1U << due_op[k];
         }
         if (job.drained()) {
@@ -143,7 +158,7 @@ __device__ __forceinline__ void pool_walk(const SceneView& s, Job& job, uint32_t
         bool due = (mine >> op & 1U) != 0U;
         int k = 0, next = entry[0];
 #pragma unroll
-        for (int j = 1; j < kPoolRays; ++j) {
+        for (int j = 1; j < kRays; ++j) {
             if (due_op[j] == op) {
                 k = j;
                 next = entry[j];
@@ -227,6 +242,49 @@ __device__ __forceinline__ void pool_walk(const SceneView& s, Job& job, uint32_t
                 ray.word(kPoolFlags) = (flags & ~kPoolSpMask) | sp;
                 after = pool_op<SPH>(next, in_world);
             }
+        } else if (ANY && op == kPoolLeaf) {
+            // the leaves' triangles, dealt evenly over the warp's lanes
+            const uint32_t packed = static_cast<uint32_t>(~next);
+            const uint32_t first = packed >> kLeafCountBits;
+            const uint32_t n = due ? (packed & (kMaxLeafSize - 1)) + 1U : 0U;
+            const uint32_t lane = threadIdx.x & 31U, below = (1U << lane) - 1U;
+            const unsigned ones = __ballot_sync(0xFFFFFFFFU, (n & 1U) != 0U);
+            const unsigned twos = __ballot_sync(0xFFFFFFFFU, (n & 2U) != 0U);
+            const unsigned fours = __ballot_sync(0xFFFFFFFFU, (n & 4U) != 0U);
+            const uint32_t from = __popc(ones & below) + 2U * __popc(twos & below) + 4U * __popc(fours & below);
+            const uint32_t total = __popc(ones) + 2U * __popc(twos) + 4U * __popc(fours);
+            uint32_t* const tests = shared + kPoolRayWords<ANY> + (threadIdx.x >> 5) * kPoolTests;
+            uint8_t* const owners =
+                reinterpret_cast<uint8_t*>(shared + kPoolRayWords<ANY> + (kPoolThreads / 32) * kPoolTests) +
+                (threadIdx.x >> 5) * kPoolTests;
+            for (uint32_t j = 0; j < n; ++j) {
+                tests[from + j] = first + j;
+                owners[from + j] = static_cast<uint8_t>(lane | static_cast<uint32_t>(k) << 5);
+            }
+            __syncwarp();
+            for (uint32_t q = lane; q < total; q += 32U) {
+                const uint32_t owner = owners[q];
+                const PoolRay asked{shared + (threadIdx.x & ~31U) + (owner & 31U) +
+                                        (owner >> 5) * (kPoolWords * kPoolThreads),
+                                    nullptr};
+                const float4* record = s.leaf_tris + 3ULL * tests[q];
+                TriangleHit th;
+                const int res = triangle_test(record[0], record[1], record[2], asked.vec(kPoolO), asked.vec(kPoolD),
+                                              asked.real(kPoolTMin), asked.real(kPoolLimit), false, th);
+                tests[q] = res == kTriHit ? 0U : (res == kTriFailure ? kPoolFailure : kPoolMiss);
+            }
+            __syncwarp();
+            if (due) {
+                uint32_t flags = ray.word(kPoolFlags);
+                uint32_t sp = flags & kPoolSpMask;
+                for (uint32_t j = 0; j < n; ++j) {
+                    const uint32_t answer = tests[from + j];
+                    flags |= answer == 0U ? kPoolFound : (answer == kPoolFailure ? kPoolFailed : 0U);
+                }
+                next = (flags & kPoolFound) != 0U ? kPoolDone : ray.pop(sp);
+                ray.word(kPoolFlags) = (flags & ~kPoolSpMask) | sp;
+                after = pool_op<SPH>(next, in_world);
+            }
         } else if (op == kPoolLeaf || (SPH && op == kPoolSphere)) {
             if (due) {
                 uint32_t flags = ray.word(kPoolFlags);
@@ -248,13 +306,13 @@ __device__ __forceinline__ void pool_walk(const SceneView& s, Job& job, uint32_t
                         r1 = record[1];
                         r2 = record[2];
                     }
-                    int res;
-                    float t;
+                    int res = kTriMiss;
+                    float t = 0.0F;
                     if (SPH && op == kPoolSphere) {
                         const SphereHit h = sphere_intersect(v0, v1.x, o, d, t_min, limit);
                         res = static_cast<int>(h.outcome);
                         t = h.t;
-                    } else {
+                    } else if constexpr (!ANY) {
                         TriangleHit th;
                         res = triangle_test(v0, v1, v2, o, d, t_min, limit, false, th);
                         t = th.t;
@@ -341,7 +399,7 @@ __device__ __forceinline__ void pool_walk(const SceneView& s, Job& job, uint32_t
         }
         if (due) {
 #pragma unroll
-            for (int j = 0; j < kPoolRays; ++j) {
+            for (int j = 0; j < kRays; ++j) {
                 entry[j] = k == j ? next : entry[j];
                 due_op[j] = k == j ? after : due_op[j];
             }
@@ -654,7 +712,7 @@ __global__ void __launch_bounds__(kPoolThreads, kPoolBlocks) k_query_occlusion(S
 
 // Launches a pool kernel over `rays` rays at most: one resident wave of blocks, or as many as give
 // every lane a ray.
-template <class... Params, class... Args>
+template <bool ANY, class... Params, class... Args>
 cudaError_t launch_pool(void (*kernel)(Params...), uint64_t rays, cudaStream_t stream, Args... args) {
     int device = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&device);
@@ -663,7 +721,7 @@ cudaError_t launch_pool(void (*kernel)(Params...), uint64_t rays, cudaStream_t s
     }
     if (e == cudaSuccess) {
         e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(kPoolSharedBytes));
+                                 static_cast<int>(kPoolSharedBytes<ANY>));
     }
     if (e != cudaSuccess) {
         return e;
@@ -671,7 +729,7 @@ cudaError_t launch_pool(void (*kernel)(Params...), uint64_t rays, cudaStream_t s
     const uint64_t wave = static_cast<uint64_t>(sms) * kPoolBlocks;
     const uint64_t need = (rays + kPoolThreads - 1U) / kPoolThreads;
     const uint32_t blocks = static_cast<uint32_t>(need < wave ? (need == 0U ? 1U : need) : wave);
-    kernel<<<blocks, kPoolThreads, kPoolSharedBytes, stream>>>(args...);
+    kernel<<<blocks, kPoolThreads, kPoolSharedBytes<ANY>, stream>>>(args...);
     return cudaGetLastError();
 }
 
