@@ -152,6 +152,88 @@ __global__ void __launch_bounds__(256) k_compact_scatter(const uint8_t* __restri
     }
 }
 
+// The same compaction by one block, each of its warps owning a run of consecutive slots: for the few
+// slots of a short trace, where the three launches above take longer than their work.
+template <uint32_t MAX>
+__global__ void __launch_bounds__(1024) k_compact_block(const uint8_t* __restrict__ keys, uint32_t n, uint32_t routes,
+                                                        uint32_t* __restrict__ queue, uint32_t* __restrict__ offsets,
+                                                        unsigned long long* __restrict__ total,
+                                                        uint8_t* __restrict__ reset_keys) {
+    __shared__ uint32_t counts[MAX][32];
+    __shared__ uint32_t route_base[MAX + 1U];
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31U;
+    const uint32_t run = (n + 1023U) / 1024U * 32U;  // slots per warp, whole groups of 32
+    const uint32_t begin = warp * run;
+    uint32_t count[MAX] = {};
+    for (uint32_t step = 0; step < run; step += 32U) {
+        const uint32_t key = key_at(keys, n, begin + step + lane);
+#pragma unroll
+        for (uint32_t r = 0; r < MAX; ++r) {
+            count[r] += __popc(__ballot_sync(0xFFFFFFFFU, key == r && r < routes));
+        }
+    }
+    if (lane == 0U) {
+#pragma unroll
+        for (uint32_t r = 0; r < MAX; ++r) {
+            counts[r][warp] = count[r];
+        }
+    }
+    __syncthreads();
+    if (warp < MAX) {  // warp r: the runs' places within route r
+        const uint32_t own = counts[warp][lane];
+        uint32_t sum = own;
+        for (uint32_t off = 1U; off < 32U; off <<= 1U) {
+            const uint32_t v = __shfl_up_sync(0xFFFFFFFFU, sum, off);
+            sum += lane >= off ? v : 0U;
+        }
+        counts[warp][lane] = sum - own;
+        if (lane == 31U) {
+            route_base[warp + 1U] = sum;
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0U) {
+        route_base[0] = 0U;
+        for (uint32_t r = 0; r < MAX; ++r) {
+            route_base[r + 1U] += route_base[r];
+        }
+        if (total != nullptr) {
+            *total = route_base[routes];
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x <= routes) {
+        offsets[threadIdx.x] = route_base[threadIdx.x];
+    }
+    uint32_t base[MAX];
+#pragma unroll
+    for (uint32_t r = 0; r < MAX; ++r) {
+        base[r] = route_base[r] + counts[r][warp];
+    }
+    const uint32_t below = (1U << lane) - 1U;
+    for (uint32_t step = 0; step < run; step += 32U) {
+        const uint32_t slot = begin + step + lane;
+        const uint32_t key = key_at(keys, n, slot);
+#pragma unroll
+        for (uint32_t r = 0; r < MAX; ++r) {
+            const bool mine = key == r && r < routes;
+            const unsigned ballot = __ballot_sync(0xFFFFFFFFU, mine);
+            if (mine) {
+                queue[base[r] + __popc(ballot & below)] = slot;
+            }
+            base[r] += __popc(ballot);
+        }
+        if (reset_keys != nullptr && slot < n) {
+            reset_keys[slot] = kRouteNone;
+        }
+    }
+}
+
+// One block up to this many slots. A plain Cornell box of one sample per pixel took 1.38 ms in three
+// launches and 1.16 ms in one block with 4,096 slots, 1.41 and 1.39 ms with 16,384, 1.50 and 1.73 ms with
+// 32,761.
+constexpr uint32_t kCompactBlockSlots = 16384U;
+
 }  // namespace
 
 cudaError_t launch_compaction(const uint8_t* keys, uint32_t n, uint32_t routes, uint32_t* tile_counts,
@@ -160,7 +242,18 @@ cudaError_t launch_compaction(const uint8_t* keys, uint32_t n, uint32_t routes, 
     if (routes == 0U || routes > kCompactMaxRoutes) {
         return cudaErrorInvalidValue;
     }
-    const uint32_t tiles = n == 0U ? 1U : (n + kCompactTile - 1U) / kCompactTile;
+    if (n <= kCompactBlockSlots) {
+        if (routes <= kCompactFewRoutes) {
+            k_compact_block<kCompactFewRoutes><<<1, 1024, 0, stream>>>(keys, n, routes, queue, offsets, total,
+                                                                      reset_keys);
+        } else {
+            k_compact_block<kCompactMaxRoutes><<<1, 1024, 0, stream>>>(keys, n, routes, queue, offsets, total,
+                                                                      reset_keys);
+        }
+        *launches += 1U;
+        return cudaGetLastError();
+    }
+    const uint32_t tiles = (n + kCompactTile - 1U) / kCompactTile;
     if (routes <= kCompactFewRoutes) {
         k_compact_count<kCompactFewRoutes><<<tiles, 256, 0, stream>>>(keys, n, routes, tiles, tile_counts);
     } else {

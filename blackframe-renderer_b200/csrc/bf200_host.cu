@@ -57,6 +57,7 @@ struct bf200_context {
     size_t film_staging_bytes = 0;
     void* batch_staging = nullptr;  // device copies of host path inputs and results, and of query rays and answers
     size_t batch_staging_bytes = 0;
+    bf200::ShadeBranches shade_branches{};
     // film batches (bf200_render_films_device): one stream, event, arena slice, pinned counter
     // block and radiance buffer per lane, kept across calls
     std::vector<cudaStream_t> lane_streams;
@@ -971,6 +972,9 @@ size_t carve_wavefront(char* base, uint32_t capacity, Wavefront* out) {
     return offset;
 }
 
+// Iteration outcomes in pinned memory behind the counters' copy (run_wavefront_streamed).
+constexpr uint32_t kOutcomes = 4U;
+
 blackframe_status ensure_capacity(bf200_context* c) {
     if (c->arena != nullptr) {
         return BLACKFRAME_STATUS_SUCCESS;
@@ -982,11 +986,29 @@ blackframe_status ensure_capacity(bf200_context* c) {
         return cuda_fail(c, e, "wavefront allocation");
     }
     carve_wavefront(static_cast<char*>(c->arena), n, &c->w);
-    e = cudaMallocHost(&c->pinned_counters, kWavefrontCounters * sizeof(unsigned long long));
+    e = cudaMallocHost(&c->pinned_counters, (kWavefrontCounters + kOutcomes) * sizeof(unsigned long long));
     if (e != cudaSuccess) {
         return cuda_fail(c, e, "pinned counters");
     }
     return BLACKFRAME_STATUS_SUCCESS;
+}
+
+// The streams and events of the shading stage's branches.
+blackframe_status ensure_shade_branches(bf200_context* c) {
+    ShadeBranches& b = c->shade_branches;
+    cudaError_t e = cudaSuccess;
+    if (b.fork == nullptr) {
+        e = cudaEventCreateWithFlags(&b.fork, cudaEventDisableTiming);
+    }
+    for (uint32_t k = 0; k < kShadeBranches && e == cudaSuccess; ++k) {
+        if (b.stream[k] == nullptr) {
+            e = cudaStreamCreateWithFlags(&b.stream[k], cudaStreamNonBlocking);
+        }
+        if (e == cudaSuccess && b.join[k] == nullptr) {
+            e = cudaEventCreateWithFlags(&b.join[k], cudaEventDisableTiming);
+        }
+    }
+    return e == cudaSuccess ? BLACKFRAME_STATUS_SUCCESS : cuda_fail(c, e, "shading branches");
 }
 
 TransportParams make_params(const bf200_transport_options_v1& o) {
@@ -1109,13 +1131,42 @@ Wavefront fit_slots(const Wavefront& w, uint64_t paths) {
     return fitted;
 }
 
-// The persistent wavefront as one CUDA graph: a conditional WHILE node whose body is one iteration
-// (the stage kernels and k_iteration_gate, which decides on the device whether another iteration
-// runs), so the whole trace is one graph launch with no host round trip per iteration. The gate
-// stops at the same iteration bound as the host loop.
-blackframe_status run_wavefront_graph(bf200_context* c, const bf200_scene* s, PathSource src,
-                                      const TransportParams& p, bf200_report_v1* report,
-                                      const AdjointView* adjoint = nullptr) {
+// Adds a finished trace's counters (their pinned copy) to the caller's report.
+void wavefront_report(const bf200_context* c, const bf200_scene* s, const PathSource& src, uint64_t iterations,
+                      uint64_t launches, bf200_report_v1* report) {
+    if (report == nullptr) {
+        return;
+    }
+    const unsigned long long* k = c->pinned_counters;
+    report->struct_size = sizeof(bf200_report_v1);
+    report->registered_light_count = s->light_count;
+    report->path_count += src.total;
+    report->extension_segments += k[3];
+    report->shadow_segments += k[4];
+    report->failed_lanes += k[5];
+    report->terminated_paths += src.total - std::min<uint64_t>(src.total, k[5]);
+    report->closure_samples += k[11];
+    report->light_samples += k[12];
+    report->miss_segments += k[13];
+    report->continuation_segments += k[14];
+    if (k[5] != 0 && report->first_failure_status == 0) {
+        report->first_failure_status = static_cast<uint32_t>(k[7]);
+        report->first_failure_path = static_cast<uint32_t>(k[6]);
+    }
+    report->kernel_launches += launches;
+    report->iterations += iterations;
+}
+
+// The persistent wavefront, its iterations queued by the host one ahead of the GPU: while iteration i + 1
+// runs, the host reads how iteration i ended from pinned memory, so the GPU does not wait for the host,
+// and one idle iteration is queued past the last. It stops at the same iteration bound as the
+// instrumented loop. One CUDA graph with a device-side loop over the iteration did the same before:
+// building, instantiating and destroying it cost each call 240 us, 430 us with the shading branches, and
+// once running it was no faster (one 1 x 1 path 706 us as a graph, 230 us so; 64 x 64 plain Cornell box
+// 1.45 and 1.10 ms; Cornell box with spheres, 256 spp, 75.8 and 75.9 ms).
+blackframe_status run_wavefront_streamed(bf200_context* c, const bf200_scene* s, PathSource src,
+                                         const TransportParams& p, bf200_report_v1* report,
+                                         const AdjointView* adjoint) {
     const Wavefront w = fit_slots(c->w, src.total);
     cudaStream_t st = c->stream;
     cudaError_t e = cudaMemsetAsync(w.state, 0, w.capacity, st);
@@ -1132,98 +1183,67 @@ blackframe_status run_wavefront_graph(bf200_context* c, const bf200_scene* s, Pa
         std::max<uint32_t>(1, std::min<uint32_t>((w.capacity + 255U) / 256U, c->sm_count * 8U));
     const uint64_t depth_bound = static_cast<uint64_t>(p.limits[0]) + p.limits[1] + p.limits[2] + 2;
     const uint64_t max_iterations = 64 + 2 * (src.total / w.capacity + 2) * depth_bound;
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
-    cudaGraphConditionalHandle loop = 0;
-    uint32_t per_iteration = 0;
-    e = cudaGraphCreate(&graph, 0);
-    if (e == cudaSuccess) {
-        e = cudaGraphConditionalHandleCreate(&loop, graph, 1U, cudaGraphCondAssignDefault);
+    volatile unsigned long long* outcomes = c->pinned_counters + kWavefrontCounters;
+    if (const auto b = ensure_shade_branches(c); b != BLACKFRAME_STATUS_SUCCESS) {
+        return b;
     }
-    cudaGraphNode_t node = nullptr;
-    cudaGraphNodeParams params{};
-    params.type = cudaGraphNodeTypeConditional;
-    params.conditional.handle = loop;
-    params.conditional.type = cudaGraphCondTypeWhile;
-    params.conditional.size = 1;
-    if (e == cudaSuccess) {
-        e = cudaGraphAddNode(&node, graph, nullptr, 0, &params);
-    }
-    if (e == cudaSuccess) {
-        cudaGraph_t body = params.conditional.phGraph_out[0];
-        e = cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
+    uint32_t launches = 0;
+    uint64_t queued = 0, ended = 0;
+    bool drained = false;
+    while (e == cudaSuccess && !drained && ended < max_iterations) {
+        outcomes[queued % kOutcomes] = 0ULL;
         for (int stage = 0; stage < 4 && e == cudaSuccess; ++stage) {
-            e = launch_stage(stage, s->view, w, src, p, grid, st, &per_iteration, adjoint);
+            e = launch_stage(stage, s->view, w, src, p, grid, st, &launches, adjoint, &c->shade_branches);
         }
         if (e == cudaSuccess) {
-            e = launch_gate(w, src.total, max_iterations, loop, st);
-            ++per_iteration;
+            e = launch_iteration_end(w, src.total, outcomes + queued % kOutcomes, st);
+            ++launches;
         }
-        cudaGraph_t captured = nullptr;
-        const cudaError_t end = cudaStreamEndCapture(st, &captured);
-        if (e == cudaSuccess) {
-            e = end;
+        if (++queued < 2U || e != cudaSuccess) {
+            continue;
         }
-    }
-    if (e == cudaSuccess) {
-        e = cudaGraphInstantiate(&exec, graph, 0);
-    }
-    if (e == cudaSuccess) {
-        e = cudaGraphLaunch(exec, st);
+        // the outcome of the iteration before the one just queued
+        for (uint32_t spins = 1U; outcomes[ended % kOutcomes] == 0ULL && e == cudaSuccess; ++spins) {
+            if (spins % 4096U != 0U) {
+                continue;
+            }
+            const cudaError_t state = cudaStreamQuery(st);
+            if (state == cudaSuccess) {  // nothing left to run: the outcome has been written
+                break;
+            }
+            e = state == cudaErrorNotReady ? cudaSuccess : state;
+        }
+        drained = e == cudaSuccess && outcomes[ended % kOutcomes] == kIterationDrained;
+        ++ended;
     }
     if (e == cudaSuccess) {
         e = launch_retire(w, src, grid, st);
     }
     if (e == cudaSuccess) {
-        e = cudaMemcpyAsync(c->pinned_counters, w.counters, kWavefrontCounters * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                            st);
+        e = cudaMemcpyAsync(c->pinned_counters, w.counters, kWavefrontCounters * sizeof(unsigned long long),
+                            cudaMemcpyDeviceToHost, st);
     }
+    const cudaError_t done = cudaStreamSynchronize(st);
     if (e == cudaSuccess) {
-        e = cudaStreamSynchronize(st);
-    }
-    if (exec != nullptr) {
-        cudaGraphExecDestroy(exec);
-    }
-    if (graph != nullptr) {
-        cudaGraphDestroy(graph);
+        e = done;
     }
     if (e != cudaSuccess) {
-        return cuda_fail(c, e, "wavefront graph");
+        return cuda_fail(c, e, "wavefront");
     }
-    const unsigned long long* k = c->pinned_counters;
-    if (k[10] != 0ULL) {
+    if (!drained) {
         return fail(c, BLACKFRAME_STATUS_INVALID_STATE, "the wavefront did not drain within its iteration bound");
     }
-    if (report != nullptr) {
-        report->struct_size = sizeof(bf200_report_v1);
-        report->registered_light_count = s->light_count;
-        report->path_count += src.total;
-        report->extension_segments += k[3];
-        report->shadow_segments += k[4];
-        report->failed_lanes += k[5];
-        report->terminated_paths += src.total - std::min<uint64_t>(src.total, k[5]);
-        report->closure_samples += k[11];
-        report->light_samples += k[12];
-        report->miss_segments += k[13];
-        report->continuation_segments += k[14];
-        if (k[5] != 0 && report->first_failure_status == 0) {
-            report->first_failure_status = static_cast<uint32_t>(k[7]);
-            report->first_failure_path = static_cast<uint32_t>(k[6]);
-        }
-        report->kernel_launches += k[9] * per_iteration + 1U;
-        report->iterations += k[9];
-    }
+    wavefront_report(c, s, src, ended, launches + 1U, report);
     return BLACKFRAME_STATUS_SUCCESS;
 }
 
-// Runs the persistent wavefront until every path of `src` has been traced and retired. Without
-// instrumentation the loop runs on the device inside one graph; with it, the host drives every
-// iteration so each stage can be timed with events (and profilers, which do not see the kernels of
-// a device-side loop, see every launch). `adjoint` makes the run a path-replay adjoint replay.
+// Runs the persistent wavefront until every path of `src` has been traced and retired. With
+// instrumentation the host waits for every iteration, so each stage can be timed with events. `adjoint`
+// makes the run a path-replay adjoint replay.
 blackframe_status run_wavefront(bf200_context* c, const bf200_scene* s, PathSource src, const TransportParams& p,
                                 bool instrument, bf200_report_v1* report, const AdjointView* adjoint = nullptr) {
     if (!instrument) {
-        return run_wavefront_graph(c, s, src, p, report, adjoint);
+        return run_wavefront_streamed(c, s, src, p, report, adjoint);
     }
     const Wavefront w = fit_slots(c->w, src.total);
     cudaStream_t st = c->stream;
@@ -1483,6 +1503,17 @@ BF200_EXPORT blackframe_status bf200_context_destroy(bf200_context* c) noexcept 
     if (c->stream != nullptr) {
         cudaStreamSynchronize(c->stream);
         cudaStreamDestroy(c->stream);
+    }
+    for (cudaStream_t st : c->shade_branches.stream) {
+        if (st != nullptr) {
+            cudaStreamDestroy(st);
+        }
+    }
+    for (cudaEvent_t ev : {c->shade_branches.fork, c->shade_branches.join[0], c->shade_branches.join[1],
+                           c->shade_branches.join[2]}) {
+        if (ev != nullptr) {
+            cudaEventDestroy(ev);
+        }
     }
     if (c->arena != nullptr) {
         cudaFree(c->arena);

@@ -14,9 +14,16 @@ cudaError_t launch_world_normals(const SceneView& s, uint32_t total, float4* out
 // stage 0: k_regenerate; 1: k_trace, k_hits; 2: route compaction, the per-route k_shade kernels, shadow
 // compaction; 3: k_occlude. Adds the number of kernels launched to *launches. With `adjoint`, the
 // shading and occlusion stages run as the path-replay adjoint's replay.
+// With `branches`, the Lambert kernel and the other shading kernels each go on a stream of their own,
+// forked and joined by the branches' events.
+constexpr uint32_t kShadeBranches = 3U;
+struct ShadeBranches {
+    cudaStream_t stream[kShadeBranches];
+    cudaEvent_t fork, join[kShadeBranches];
+};
 cudaError_t launch_stage(int stage, const SceneView& s, const Wavefront& w, const PathSource& src,
                          const TransportParams& p, uint32_t grid, cudaStream_t stream, uint32_t* launches,
-                         const AdjointView* adjoint = nullptr);
+                         const AdjointView* adjoint = nullptr, const ShadeBranches* branches = nullptr);
 // Stable compaction of n one-byte keys: the indices whose key is r < routes go to
 // queue[offsets[r] .. offsets[r + 1]) in increasing order. tile_counts holds routes x
 // ceil(n / kCompactTile) words of scratch. When total is given it receives the queue length; when
@@ -30,12 +37,12 @@ cudaError_t launch_compaction(const uint8_t* keys, uint32_t n, uint32_t routes, 
 cudaError_t build_blas_lbvh(const float* positions, uint32_t vertex_count, const uint32_t* triangles, uint32_t n,
                             uint32_t node_base, uint32_t leaf_base, std::vector<BvhNode>& nodes,
                             std::vector<float4>& leaf_tris, cudaStream_t stream);
-// Queues k_iteration_gate, which ends one iteration of a graph's device-side wavefront loop: it
-// accumulates the shadow segments (counters[4]), counts iterations (counters[9]), clears the
-// per-iteration counters and sets `loop` to continue until the wavefront drains or
-// `max_iterations` is reached (then counters[10] = 1).
-cudaError_t launch_gate(const Wavefront& w, uint64_t total, uint64_t max_iterations, cudaGraphConditionalHandle loop,
-                        cudaStream_t stream);
+// Queues k_iteration_end, which ends one iteration of the loop that the host queues: it accumulates the
+// shadow segments (counters[4]), counts iterations (counters[9]), clears the per-iteration counters and
+// writes kIterationMore or kIterationDrained to *outcome, in pinned host memory.
+constexpr unsigned long long kIterationMore = 1ULL, kIterationDrained = 2ULL;
+cudaError_t launch_iteration_end(const Wavefront& w, uint64_t total, volatile unsigned long long* outcome,
+                                 cudaStream_t stream);
 // Retires the slots the last iteration finished (k_regenerate; nothing is left to claim).
 cudaError_t launch_retire(const Wavefront& w, const PathSource& src, uint32_t grid, cudaStream_t stream);
 cudaError_t launch_film(const float4* path_radiance, uint32_t pixels, uint32_t samples, const float* response12,

@@ -3,5 +3,5 @@
 
 namespace bf200 {
 template void launch_shade_others<false, false, true>(const SceneView&, const Wavefront&, const PathSource&, const TransportParams&,
-                                    uint32_t, const AdjointView&, cudaStream_t);
+                                    uint32_t, const AdjointView&, const cudaStream_t (&)[kShadeBranches]);
 }  // namespace bf200

@@ -53,3 +53,22 @@ def test_paths_of_many_closure_sequences_match_the_oracle(count):
     keep = want["lane_status"] == 0
     assert keep.mean() > 0.99 and got["radiance"][keep].any()
     check_paths({k: v[keep] for k, v in got.items()}, {k: v[keep] for k, v in want.items()}, f"{count} sequences")
+
+
+@pytest.mark.parametrize("n", [0, 1, 31, 33, 1023, 1024, 1025, 16383, 16384, 16385])
+@pytest.mark.parametrize("routes", [1, 3, 4])
+def test_one_block_compaction_keeps_slot_order(n, routes):
+    """Queues of up to 16,384 slots come from one block, longer ones from three launches."""
+    import torch
+    rng = np.random.default_rng(n + routes)
+    keys = rng.choice(np.array([*range(routes), 0xFF], np.uint8), max(n, 1))
+    device = torch.from_numpy(keys).cuda()
+    queue = torch.full((max(n, 1),), -1, dtype=torch.int32, device="cuda")
+    offsets = torch.zeros(routes + 1, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    with runtime.Context(0, path_capacity=1 << 12) as ctx:
+        ctx.compact_routes_device(device.data_ptr(), n, routes, queue.data_ptr(), offsets.data_ptr())
+    wanted = [np.nonzero(keys[:n] == r)[0] for r in range(routes)]
+    ends = np.cumsum([0] + [len(w) for w in wanted])
+    assert np.array_equal(offsets.cpu().numpy(), ends)
+    assert np.array_equal(queue.cpu().numpy()[:ends[-1]], np.concatenate(wanted))
