@@ -893,6 +893,20 @@ static __device__ bool transform_position_with_error(const SceneView& s, uint32_
     return true;
 }
 
+// robust_transformed_normal's scaling and division (:252-295); false when not representable.
+BF_SHARED bool divided_normal(double x, double y, double z, F3& ns) {
+    double mc = fabs(x);
+    mc = mc < fabs(y) ? fabs(y) : mc;
+    mc = mc < fabs(z) ? fabs(z) : mc;
+    if (!isfinite(mc) || mc == 0.0) {
+        return false;
+    }
+    const double sc[3] = {x / mc, y / mc, z / mc};
+    const double mag = sqrt(fma(sc[0], sc[0], fma(sc[1], sc[1], sc[2] * sc[2])));
+    ns = F3{__double2float_rn(sc[0] / mag), __double2float_rn(sc[1] / mag), __double2float_rn(sc[2] / mag)};
+    return true;
+}
+
 // robust_transformed_normal (:252-295): an object-space normal through the inverse transpose, in
 // double, scaled by its largest component and normalised.
 static __device__ bool transform_normal(const SceneView& s, uint32_t inst, F3 on, F3& ns, Lane& lane) {
@@ -921,16 +935,10 @@ static __device__ bool transform_normal(const SceneView& s, uint32_t inst, F3 on
             return true;
         }
     }
-    double mc = fabs(tr[0]);
-    mc = mc < fabs(tr[1]) ? fabs(tr[1]) : mc;
-    mc = mc < fabs(tr[2]) ? fabs(tr[2]) : mc;
-    if (!isfinite(mc) || mc == 0.0) {
+    if (!divided_normal(tr[0], tr[1], tr[2], ns)) {
         lane.fail();
         return false;
     }
-    const double sc[3] = {tr[0] / mc, tr[1] / mc, tr[2] / mc};
-    const double mag = sqrt(fma(sc[0], sc[0], fma(sc[1], sc[1], sc[2] * sc[2])));
-    ns = F3{__double2float_rn(sc[0] / mag), __double2float_rn(sc[1] / mag), __double2float_rn(sc[2] / mag)};
     return true;
 }
 
@@ -1161,8 +1169,34 @@ static __device__ void sample_mesh_light(const SceneView& s, const LightInfo& li
     out.valid = !black && lane.err == 0;
 }
 
+// scale_radiometric_value's exponent-split form: `value` times the first n numerator factors over den.
+BF_SHARED float split_radiometric(float value, int n, const Factors<3, 3> f, Lane& lane) {
+    int exponent = 0;
+    float fraction = frexpf(value, &exponent);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        int e = 0;
+        const float scaled = fraction * frexpf(f.num[i], &e);
+        fraction = i < n ? scaled : fraction;
+        exponent += i < n ? e : 0;
+    }
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        int e = 0;
+        fraction /= frexpf(f.den[i], &e);
+        exponent -= e;
+    }
+    int ne = 0;
+    fraction = frexpf(fraction, &ne);
+    const float result = scalbnf(fraction, exponent + ne);
+    if (!isfinite(result) || !(result > 0.0F)) {
+        lane.fail();
+    }
+    return result;
+}
+
 // scale_radiometric_value (PunctualLights.hpp:131-183) with n numerator and three denominator factors
-__device__ __forceinline__ float scale_radiometric(float value, const float* num, int n, const float (&den)[3],
+__device__ __forceinline__ float scale_radiometric(float value, const float (&num)[3], int n, const float (&den)[3],
                                                    Lane& lane) {
     if (!isfinite(value) || value < 0.0F) {
         lane.fail();
@@ -1199,32 +1233,12 @@ __device__ __forceinline__ float scale_radiometric(float value, const float* num
             return direct;
         }
     }
-    int exponent = 0;
-    float fraction = frexpf(value, &exponent);
-    int accumulated = exponent;
-    for (int i = 0; i < n; ++i) {
-        int e = 0;
-        fraction *= frexpf(num[i], &e);
-        accumulated += e;
-    }
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        int e = 0;
-        fraction /= frexpf(den[i], &e);
-        accumulated -= e;
-    }
-    int ne = 0;
-    fraction = frexpf(fraction, &ne);
-    const float result = scalbnf(fraction, accumulated + ne);
-    if (!isfinite(result) || !(result > 0.0F)) {
-        lane.fail();
-    }
-    return result;
+    return split_radiometric(value, n, Factors<3, 3>({num[0], num[1], num[2]}, den), lane);
 }
 
 // PointLight / DirectionalLight / SpotLight::sample_li (PunctualLights.hpp:390-430, 510-530,
 // 654-720) with IncidentLightSample::create_finite / create_infinite (Light.hpp:404-456).
-static __device__ void sample_punctual_light(const PunctualLight& light, F3 context, float u, float v,
+BF_SHARED void sample_punctual_light(const PunctualLight& light, F3 context, float u, float v,
                                              LightSample& out, Lane& lane) {
     out.valid = false;
     out.pdf = 1.0F;
@@ -1423,6 +1437,39 @@ static __device__ void mix_filter(const SceneView& s, uint32_t material, const T
 // k_shade: one bounce of the scalar MIS loop (SceneMisPathLoop.cpp:685-916) per active slot
 // ------------------------------------------------------------------------------------------------
 
+// The throughput's exponent-split form: beta * value * cosine * correction / pdf.
+BF_SHARED float split_throughput(const Factors<4, 1> f, Lane& lane) {
+    float significand = 1.0F;
+    int exponent = 0;
+    bool zero = false;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        if (!isfinite(f.num[k]) || f.num[k] < 0.0F) {
+            lane.fail();
+        }
+        if (f.num[k] == 0.0F) {
+            zero = true;
+        }
+        if (!zero) {
+            int fe = 0;
+            significand *= frexpf(f.num[k], &fe);
+            exponent += fe;
+        }
+    }
+    if (zero) {
+        return 0.0F;
+    }
+    int pe = 0, ne = 0;
+    significand /= frexpf(f.den[0], &pe);
+    exponent -= pe;
+    significand = frexpf(significand, &ne);
+    const float result = scalbnf(significand, exponent + ne);
+    if (!isfinite(result) || !(result > 0.0F)) {
+        lane.fail();
+    }
+    return result;
+}
+
 struct ShadowRecord {
     bool valid;
     F3 origin, direction;
@@ -1452,6 +1499,17 @@ __device__ __forceinline__ void add_product(float4& acc, const float4 a, const f
     acc = make_float4(r[0], r[1], r[2], r[3]);
 }
 
+BF_SHARED float split_emission(float beta, float le, float weight, Lane& lane) {
+    int e1 = 0, e2 = 0, e3 = 0, en = 0;
+    const float significand = frexpf(beta, &e1) * frexpf(le, &e2) * frexpf(weight, &e3);
+    const float normalized = frexpf(significand, &en);
+    const float contribution = scalbnf(normalized, e1 + e2 + e3 + en);
+    if (!isfinite(contribution) || !(contribution > 0.0F)) {
+        lane.fail();
+    }
+    return contribution;
+}
+
 // SceneMisPathLoop.cpp:481-528
 __device__ __forceinline__ void add_weighted_emission(float4& acc, const float4 beta, const float (&le)[4], float wgt,
                                                       Lane& lane) {
@@ -1477,13 +1535,7 @@ __device__ __forceinline__ void add_weighted_emission(float4& acc, const float4 
             r[l] = r[l] + direct;
             continue;
         }
-        int e1 = 0, e2 = 0, e3 = 0, en = 0;
-        const float significand = frexpf(bv[l], &e1) * frexpf(le[l], &e2) * frexpf(wgt, &e3);
-        const float normalized = frexpf(significand, &en);
-        const float contribution = scalbnf(normalized, e1 + e2 + e3 + en);
-        if (!isfinite(contribution) || !(contribution > 0.0F)) {
-            lane.fail();
-        }
+        const float contribution = split_emission(bv[l], le[l], wgt, lane);
         r[l] = r[l] + contribution;
     }
     acc = make_float4(r[0], r[1], r[2], r[3]);
@@ -2040,35 +2092,7 @@ __global__ void __launch_bounds__(256, BF200_SHADE_MIN_BLOCKS) k_shade(SceneView
                                     if (Factors<4, 1>(num, den).direct(nb[l])) {
                                         continue;
                                     }
-                                    float significand = 1.0F;
-                                    int exponent = 0;
-                                    bool zero = false;
-#pragma unroll
-                                    for (int k = 0; k < 4; ++k) {
-                                        if (!isfinite(num[k]) || num[k] < 0.0F) {
-                                            lane.fail();
-                                        }
-                                        if (num[k] == 0.0F) {
-                                            zero = true;
-                                        }
-                                        if (!zero) {
-                                            int fe = 0;
-                                            significand *= frexpf(num[k], &fe);
-                                            exponent += fe;
-                                        }
-                                    }
-                                    if (zero) {
-                                        nb[l] = 0.0F;
-                                        continue;
-                                    }
-                                    int pe = 0, ne = 0;
-                                    significand /= frexpf(bs.pdf, &pe);
-                                    exponent -= pe;
-                                    significand = frexpf(significand, &ne);
-                                    nb[l] = scalbnf(significand, exponent + ne);
-                                    if (!isfinite(nb[l]) || !(nb[l] > 0.0F)) {
-                                        lane.fail();
-                                    }
+                                    nb[l] = split_throughput(Factors<4, 1>(num, den), lane);
                                 }
                             }
                             const float next_eta = eta * bs.eta_scale;
@@ -2211,6 +2235,13 @@ struct SensorView {
     float normalization;
 };
 
+BF_SHARED float split_sensor_term(float c, float r, float n, float p) {
+    int ec = 0, er = 0, en = 0, ep = 0;
+    const float mc = frexpf(c, &ec), mr = frexpf(r, &er), mn = frexpf(n, &en), mp = frexpf(p, &ep);
+    const float mantissa = mc * mr * mn / mp;
+    return ldexpf(mantissa, ec + er + en - ep);
+}
+
 __device__ __forceinline__ float sensor_term(float c, float r, float n, float p) {
     if (c == 0.0F || r == 0.0F) {
         return 0.0F;
@@ -2220,10 +2251,7 @@ __device__ __forceinline__ float sensor_term(float c, float r, float n, float p)
     if (Factors<3, 1>(num, den).direct(direct)) {
         return direct;
     }
-    int ec = 0, er = 0, en = 0, ep = 0;
-    const float mc = frexpf(c, &ec), mr = frexpf(r, &er), mn = frexpf(n, &en), mp = frexpf(p, &ep);
-    const float mantissa = mc * mr * mn / mp;
-    return ldexpf(mantissa, ec + er + en - ep);
+    return split_sensor_term(c, r, n, p);
 }
 
 __global__ void k_film(const float4* path_radiance, uint32_t pixels, uint32_t samples, SensorView sensor,

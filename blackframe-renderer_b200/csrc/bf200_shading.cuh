@@ -13,7 +13,10 @@
 // One out-of-line copy of a function that the shading kernels call from several places. With every
 // call inlined the kernels were 284 KB (Lambert) to 1 MB (generic) of code, far beyond the
 // instruction cache, and their warps waited for instructions (no_instruction stalls per issue:
-// 2.6 Lambert, 10 conductor, 8 dielectric, 65 generic).
+// 2.6 Lambert, 10 conductor, 8 dielectric, 65 generic). So are the forms that few calls take
+// (the split_* products, next_of_nonfinite, divided_normal): with those inlined beside the plain ones,
+// shading took 34.0 ms (Cornell box with spheres, 256 spp) and 38.6 ms (BVH-stress frame, 16 samples), out of line
+// 32.6 and 36.4 ms.
 #define BF_SHARED static __device__ __noinline__
 // The same for the small vector and product blocks, except in the Lambert kernels (BF_SHADE_INLINE):
 // they call few of them, fit well enough, and lose more to the calls' register moves than they gain
@@ -278,9 +281,11 @@ __device__ __forceinline__ Frame rotated_about_normal(const Frame& f, float angl
 }
 
 // The next float above (up) or below: one step of the bit pattern for finite values.
+BF_SHARED float next_of_nonfinite(float value, bool up) { return nextafterf(value, up ? kInf : -kInf); }
+
 __device__ __forceinline__ float next_float(float value, bool up) {
     if (!isfinite(value)) {
-        return nextafterf(value, up ? kInf : -kInf);
+        return next_of_nonfinite(value, up);
     }
     if (value == 0.0F) {
         return up ? kDenormMin : -kDenormMin;
@@ -502,15 +507,8 @@ __device__ __forceinline__ float checked_product_ratio(const float (&num)[NN], c
     return f.direct(result) ? result : factors_ratio(f, lane);
 }
 
-// MisHeuristics.hpp:142-172
-__device__ __forceinline__ float positive_product2(float a, float b, Lane& lane) {
-    if (b == 0.0F) {
-        return 0.0F;
-    }
-    const float direct = a * b;
-    if (fminf(fminf(a, b), direct) >= kMinNormal && direct <= kMaxFloat) {
-        return direct;
-    }
+// The exponent-split product of two positive factors.
+BF_SHARED float split_product2(float a, float b, Lane& lane) {
     int ea = 0, eb = 0, en = 0;
     const float sa = frexpf(a, &ea);
     const float sb = frexpf(b, &eb);
@@ -520,6 +518,26 @@ __device__ __forceinline__ float positive_product2(float a, float b, Lane& lane)
         lane.fail();
     }
     return r;
+}
+
+// MisHeuristics.hpp:142-172
+__device__ __forceinline__ float positive_product2(float a, float b, Lane& lane) {
+    if (b == 0.0F) {
+        return 0.0F;
+    }
+    const float direct = a * b;
+    if (fminf(fminf(a, b), direct) >= kMinNormal && direct <= kMaxFloat) {
+        return direct;
+    }
+    return split_product2(a, b, lane);
+}
+
+BF_SHARED float split_mis_ratio(uint32_t heuristic, float n, float d) {
+    int ne = 0, de = 0;
+    const float ns = frexpf(n, &ne);
+    const float ds = frexpf(d, &de);
+    const float r = ns / ds;
+    return heuristic == 0U ? scalbnf(r, ne - de) : scalbnf(r * r, 2 * (ne - de));
 }
 
 // MisHeuristics.hpp:44-141
@@ -537,11 +555,7 @@ __device__ __forceinline__ float mis_weight(uint32_t heuristic, float sampled, f
     const float plain = n / d;  // at most 1
     float ratio = heuristic == 0U ? plain : plain * plain;
     if (!(fminf(fminf(n, plain), ratio) >= kMinNormal)) {
-        int ne = 0, de = 0;
-        const float ns = frexpf(n, &ne);
-        const float ds = frexpf(d, &de);
-        const float r = ns / ds;
-        ratio = heuristic == 0U ? scalbnf(r, ne - de) : scalbnf(r * r, 2 * (ne - de));
+        ratio = split_mis_ratio(heuristic, n, d);
     }
     if (small) {
         if (!(ratio > 0.0F)) {
@@ -606,6 +620,22 @@ __device__ __forceinline__ int emission_side(F3 ng, F3 wo, Lane& lane) {
     return alignment > 0.0F ? 1 : 0;
 }
 
+BF_SHARED float split_solid_angle_pdf(float area_pdf, float scale, float cubed, float alignment, Lane& lane) {
+    int es = 0, ed = 0, ec = 0, ea = 0, en = 0;
+    const float fs = frexpf(area_pdf, &es);
+    const float fd = frexpf(scale, &ed);
+    const float fc = frexpf(cubed, &ec);
+    const float fa = frexpf(alignment, &ea);
+    const float combined = fs * fd * fd * fc / fa;
+    const int exponent = es + 2 * ed + ec - ea;
+    const float normalized = frexpf(combined, &en);
+    const float converted = scalbnf(normalized, exponent + en);
+    if (!isfinite(converted) || !(converted > 0.0F)) {
+        lane.fail();
+    }
+    return converted;
+}
+
 __device__ __forceinline__ float area_to_solid_angle(float area_pdf, F3 ref, F3 surf, F3 ng, Lane& lane) {
     if (!unit_normal(ng)) {
         lane.fail();
@@ -644,19 +674,7 @@ __device__ __forceinline__ float area_to_solid_angle(float area_pdf, F3 ref, F3 
             return direct;
         }
     }
-    int es = 0, ed = 0, ec = 0, ea = 0, en = 0;
-    const float fs = frexpf(area_pdf, &es);
-    const float fd = frexpf(scale, &ed);
-    const float fc = frexpf(cubed, &ec);
-    const float fa = frexpf(alignment, &ea);
-    const float combined = fs * fd * fd * fc / fa;
-    const int exponent = es + 2 * ed + ec - ea;
-    const float normalized = frexpf(combined, &en);
-    const float converted = scalbnf(normalized, exponent + en);
-    if (!isfinite(converted) || !(converted > 0.0F)) {
-        lane.fail();
-    }
-    return converted;
+    return split_solid_angle_pdf(area_pdf, scale, cubed, alignment, lane);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -2074,14 +2092,7 @@ __device__ __forceinline__ float positive_probability_product(float selection, f
     if (fminf(fminf(selection, conditional), direct) >= kMinNormal && direct <= kMaxFloat) {
         return direct;
     }
-    int se = 0, ce = 0, ne = 0;
-    const float ss = frexpf(selection, &se), cs = frexpf(conditional, &ce);
-    const float normalized = frexpf(ss * cs, &ne);
-    const float product = scalbnf(normalized, se + ce + ne);
-    if (!isfinite(product) || !(product > 0.0F)) {
-        lane.fail();
-    }
-    return product;
+    return split_product2(selection, conditional, lane);
 }
 
 // mix_probability_densities (ClosureMixture.hpp:270-334)
