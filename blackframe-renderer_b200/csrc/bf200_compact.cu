@@ -29,10 +29,13 @@ __device__ __forceinline__ uint32_t key_at(const uint8_t* keys, uint32_t n, uint
 
 // MAX: compiled route limit (4 for the shadow queue, the sort and the public call, kCompactMaxRoutes
 // for shading), so that few routes do not pay for the ballots of many.
+// The kernels read what the launch before them writes, and a chained launch may start while that one runs:
+// so their inputs are not declared read-only for the whole kernel (no __restrict__ on a const pointer).
 template <uint32_t MAX>
-__global__ void __launch_bounds__(256) k_compact_count(const uint8_t* __restrict__ keys, uint32_t n, uint32_t routes,
+__global__ void __launch_bounds__(256) k_compact_count(const uint8_t* keys, uint32_t n, uint32_t routes,
                                                        uint32_t tiles, uint32_t* __restrict__ tile_counts) {
     __shared__ uint32_t partial[kCompactWarps][MAX];
+    chain_begin();
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31U;
     const uint32_t first = blockIdx.x * kCompactTile + warp * kWarpSlots;
     uint32_t count[MAX] = {};
@@ -64,6 +67,7 @@ __global__ void __launch_bounds__(kScanThreads) k_compact_scan(uint32_t* __restr
                                                                uint32_t tiles, uint32_t* __restrict__ offsets,
                                                                unsigned long long* __restrict__ total) {
     __shared__ uint32_t sums[kScanThreads];
+    chain_begin();
     const uint32_t m = routes * tiles;
     const uint32_t per = (m + kScanThreads - 1U) / kScanThreads;
     const uint32_t begin = threadIdx.x * per;
@@ -96,11 +100,12 @@ __global__ void __launch_bounds__(kScanThreads) k_compact_scan(uint32_t* __restr
 }
 
 template <uint32_t MAX>
-__global__ void __launch_bounds__(256) k_compact_scatter(const uint8_t* __restrict__ keys, uint32_t n,
+__global__ void __launch_bounds__(256) k_compact_scatter(const uint8_t* keys, uint32_t n,
                                                          uint32_t routes, uint32_t tiles,
-                                                         const uint32_t* __restrict__ tile_offsets,
+                                                         const uint32_t* tile_offsets,
                                                          uint32_t* __restrict__ queue, uint8_t* __restrict__ reset_keys) {
     __shared__ uint32_t warp_base[kCompactWarps][MAX];
+    chain_begin();
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31U;
     const uint32_t first = blockIdx.x * kCompactTile + warp * kWarpSlots;
     uint32_t count[MAX] = {};
@@ -155,12 +160,13 @@ __global__ void __launch_bounds__(256) k_compact_scatter(const uint8_t* __restri
 // The same compaction by one block, each of its warps owning a run of consecutive slots: for the few
 // slots of a short trace, where the three launches above take longer than their work.
 template <uint32_t MAX>
-__global__ void __launch_bounds__(1024) k_compact_block(const uint8_t* __restrict__ keys, uint32_t n, uint32_t routes,
+__global__ void __launch_bounds__(1024) k_compact_block(const uint8_t* keys, uint32_t n, uint32_t routes,
                                                         uint32_t* __restrict__ queue, uint32_t* __restrict__ offsets,
                                                         unsigned long long* __restrict__ total,
                                                         uint8_t* __restrict__ reset_keys) {
     __shared__ uint32_t counts[MAX][32];
     __shared__ uint32_t route_base[MAX + 1U];
+    chain_begin();
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31U;
     const uint32_t run = (n + 1023U) / 1024U * 32U;  // slots per warp, whole groups of 32
     const uint32_t begin = warp * run;
@@ -238,37 +244,35 @@ constexpr uint32_t kCompactBlockSlots = 16384U;
 
 cudaError_t launch_compaction(const uint8_t* keys, uint32_t n, uint32_t routes, uint32_t* tile_counts,
                               uint32_t* queue, uint32_t* offsets, unsigned long long* total, uint8_t* reset_keys,
-                              cudaStream_t stream, uint32_t* launches) {
+                              cudaStream_t stream, uint32_t* launches, bool chained) {
     if (routes == 0U || routes > kCompactMaxRoutes) {
         return cudaErrorInvalidValue;
     }
     if (n <= kCompactBlockSlots) {
-        if (routes <= kCompactFewRoutes) {
-            k_compact_block<kCompactFewRoutes><<<1, 1024, 0, stream>>>(keys, n, routes, queue, offsets, total,
-                                                                      reset_keys);
-        } else {
-            k_compact_block<kCompactMaxRoutes><<<1, 1024, 0, stream>>>(keys, n, routes, queue, offsets, total,
-                                                                      reset_keys);
-        }
         *launches += 1U;
-        return cudaGetLastError();
+        return routes <= kCompactFewRoutes
+                   ? launch_chained(k_compact_block<kCompactFewRoutes>, 1U, 1024U, 0, stream, chained, keys, n, routes, queue,
+                                    offsets, total, reset_keys)
+                   : launch_chained(k_compact_block<kCompactMaxRoutes>, 1U, 1024U, 0, stream, chained, keys, n, routes, queue,
+                                    offsets, total, reset_keys);
     }
     const uint32_t tiles = (n + kCompactTile - 1U) / kCompactTile;
-    if (routes <= kCompactFewRoutes) {
-        k_compact_count<kCompactFewRoutes><<<tiles, 256, 0, stream>>>(keys, n, routes, tiles, tile_counts);
-    } else {
-        k_compact_count<kCompactMaxRoutes><<<tiles, 256, 0, stream>>>(keys, n, routes, tiles, tile_counts);
-    }
-    k_compact_scan<<<1, kScanThreads, 0, stream>>>(tile_counts, routes, tiles, offsets, total);
-    if (routes <= kCompactFewRoutes) {
-        k_compact_scatter<kCompactFewRoutes>
-            <<<tiles, 256, 0, stream>>>(keys, n, routes, tiles, tile_counts, queue, reset_keys);
-    } else {
-        k_compact_scatter<kCompactMaxRoutes>
-            <<<tiles, 256, 0, stream>>>(keys, n, routes, tiles, tile_counts, queue, reset_keys);
-    }
     *launches += 3U;
-    return cudaGetLastError();
+    cudaError_t e = routes <= kCompactFewRoutes ? launch_chained(k_compact_count<kCompactFewRoutes>, tiles, 256U, 0, stream, chained, keys, n,
+                                                     routes, tiles, tile_counts)
+                                    : launch_chained(k_compact_count<kCompactMaxRoutes>, tiles, 256U, 0, stream, chained, keys, n,
+                                                     routes, tiles, tile_counts);
+    if (e == cudaSuccess) {
+        e = launch_chained(k_compact_scan, 1U, kScanThreads, 0, stream, chained, tile_counts, routes, tiles, offsets, total);
+    }
+    if (e != cudaSuccess) {
+        return e;
+    }
+    return routes <= kCompactFewRoutes
+               ? launch_chained(k_compact_scatter<kCompactFewRoutes>, tiles, 256U, 0, stream, chained, keys, n, routes, tiles,
+                                tile_counts, queue, reset_keys)
+               : launch_chained(k_compact_scatter<kCompactMaxRoutes>, tiles, 256U, 0, stream, chained, keys, n, routes, tiles,
+                                tile_counts, queue, reset_keys);
 }
 
 }  // namespace bf200

@@ -1183,6 +1183,7 @@ blackframe_status run_wavefront_streamed(bf200_context* c, const bf200_scene* s,
         std::max<uint32_t>(1, std::min<uint32_t>((w.capacity + 255U) / 256U, c->sm_count * 8U));
     const uint64_t depth_bound = static_cast<uint64_t>(p.limits[0]) + p.limits[1] + p.limits[2] + 2;
     const uint64_t max_iterations = 64 + 2 * (src.total / w.capacity + 2) * depth_bound;
+    const bool chained = w.capacity <= kChainSlots;
     volatile unsigned long long* outcomes = c->pinned_counters + kWavefrontCounters;
     if (const auto b = ensure_shade_branches(c); b != BLACKFRAME_STATUS_SUCCESS) {
         return b;
@@ -1193,10 +1194,10 @@ blackframe_status run_wavefront_streamed(bf200_context* c, const bf200_scene* s,
     while (e == cudaSuccess && !drained && ended < max_iterations) {
         outcomes[queued % kOutcomes] = 0ULL;
         for (int stage = 0; stage < 4 && e == cudaSuccess; ++stage) {
-            e = launch_stage(stage, s->view, w, src, p, grid, st, &launches, adjoint, &c->shade_branches);
+            e = launch_stage(stage, s->view, w, src, p, grid, st, &launches, adjoint, &c->shade_branches, chained);
         }
         if (e == cudaSuccess) {
-            e = launch_iteration_end(w, src.total, outcomes + queued % kOutcomes, st);
+            e = launch_iteration_end(w, src.total, outcomes + queued % kOutcomes, st, chained);
             ++launches;
         }
         if (++queued < 2U || e != cudaSuccess) {

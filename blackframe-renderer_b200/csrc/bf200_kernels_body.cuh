@@ -797,6 +797,7 @@ __device__ __forceinline__ unsigned long long reserve(unsigned long long* counte
 __global__ void __launch_bounds__(256) k_regenerate(Wavefront w, PathSource src) {
     __shared__ uint32_t claim_counts[8], queue_counts[8];
     __shared__ unsigned long long claim_base, queue_base;
+    chain_begin();
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         w.counters[kCounterTraceCursor] = 0ULL;
         w.counters[kCounterOccludeCursor] = 0ULL;
@@ -2446,6 +2447,7 @@ cudaError_t launch_shading(const SceneView& s, const Wavefront& w, const PathSou
 // per-iteration counters for the next one and tells the host (pinned memory) whether every path has
 // been traced.
 __global__ void k_iteration_end(Wavefront w, uint64_t total, volatile unsigned long long* outcome) {
+    chain_begin();
     unsigned long long* c = w.counters;
     c[4] += c[0];
     ++c[9];
@@ -2461,9 +2463,8 @@ __global__ void k_iteration_end(Wavefront w, uint64_t total, volatile unsigned l
 // ------------------------------------------------------------------------------------------------
 
 cudaError_t launch_iteration_end(const Wavefront& w, uint64_t total, volatile unsigned long long* outcome,
-                                 cudaStream_t stream) {
-    k_iteration_end<<<1, 1, 0, stream>>>(w, total, outcome);
-    return cudaGetLastError();
+                                 cudaStream_t stream, bool chained) {
+    return launch_chained(k_iteration_end, 1U, 1U, 0, stream, chained, w, total, outcome);
 }
 
 cudaError_t launch_world_normals(const SceneView& s, uint32_t total, float4* out, uint32_t* failures,
@@ -2478,32 +2479,31 @@ cudaError_t launch_world_normals(const SceneView& s, uint32_t total, float4* out
 
 cudaError_t launch_stage(int stage, const SceneView& s, const Wavefront& w, const PathSource& src,
                          const TransportParams& p, uint32_t grid, cudaStream_t stream, uint32_t* launches,
-                         const AdjointView* adjoint, const ShadeBranches* branches) {
+                         const AdjointView* adjoint, const ShadeBranches* branches, bool chained) {
     cudaError_t e = cudaSuccess;
     if (stage == 0) {
-        k_regenerate<<<grid, 256, 0, stream>>>(w, src);
         *launches += 1U;
-        return cudaGetLastError();
+        return launch_chained(k_regenerate, grid, 256U, 0, stream, chained, w, src);
     }
     if (stage == 1) {
         *launches += 2U;
         if (s.sphere_count != 0U) {
-            e = launch_pool<false>(k_trace<true>, w.capacity, stream, s, w);
+            e = launch_pool<false>(k_trace<true>, w.capacity, stream, chained, s, w);
             if (e == cudaSuccess) {
-                k_hits<true><<<grid, 256, 0, stream>>>(s, w);
+                e = launch_chained(k_hits<true>, grid, 256U, 0, stream, chained, s, w);
             }
         } else {
-            e = launch_pool<false>(k_trace<false>, w.capacity, stream, s, w);
+            e = launch_pool<false>(k_trace<false>, w.capacity, stream, chained, s, w);
             if (e == cudaSuccess) {
-                k_hits<false><<<grid, 256, 0, stream>>>(s, w);
+                e = launch_chained(k_hits<false>, grid, 256U, 0, stream, chained, s, w);
             }
         }
-        return e == cudaSuccess ? cudaGetLastError() : e;
+        return e;
     }
     if (stage == 2) {
         // route the traced slots, shade each route with its own kernel, then queue the shadow rays
         e = launch_compaction(w.route, w.capacity, kRouteCount, w.tile_counts, w.route_queue, w.route_offsets,
-                              nullptr, w.shadow_key, stream, launches);
+                              nullptr, w.shadow_key, stream, launches, chained);
         if (e != cudaSuccess) {
             return e;
         }
@@ -2525,21 +2525,20 @@ cudaError_t launch_stage(int stage, const SceneView& s, const Wavefront& w, cons
             return e;
         }
         return launch_compaction(w.shadow_key, w.capacity, 1U, w.tile_counts, w.shadow_queue, w.shadow_offsets,
-                                 w.counters + 0, nullptr, stream, launches);
+                                 w.counters + 0, nullptr, stream, launches, chained);
     }
     const AdjointView a = adjoint != nullptr ? *adjoint : AdjointView{};
     *launches += 1U;
     if (s.sphere_count != 0U) {
-        return adjoint != nullptr ? launch_pool<true>(k_occlude<true, true>, w.capacity, stream, s, w, a)
-                                  : launch_pool<true>(k_occlude<false, true>, w.capacity, stream, s, w, a);
+        return adjoint != nullptr ? launch_pool<true>(k_occlude<true, true>, w.capacity, stream, chained, s, w, a)
+                                  : launch_pool<true>(k_occlude<false, true>, w.capacity, stream, chained, s, w, a);
     }
-    return adjoint != nullptr ? launch_pool<true>(k_occlude<true, false>, w.capacity, stream, s, w, a)
-                              : launch_pool<true>(k_occlude<false, false>, w.capacity, stream, s, w, a);
+    return adjoint != nullptr ? launch_pool<true>(k_occlude<true, false>, w.capacity, stream, chained, s, w, a)
+                              : launch_pool<true>(k_occlude<false, false>, w.capacity, stream, chained, s, w, a);
 }
 
 cudaError_t launch_retire(const Wavefront& w, const PathSource& src, uint32_t grid, cudaStream_t stream) {
-    k_regenerate<<<grid, 256, 0, stream>>>(w, src);
-    return cudaGetLastError();
+    return launch_chained(k_regenerate, grid, 256U, 0, stream, false, w, src);
 }
 
 cudaError_t launch_film(const float4* path_radiance, uint32_t pixels, uint32_t samples, const float* response12,
@@ -2569,8 +2568,8 @@ cudaError_t launch_adjoint_image(const float4* film32, const double* film64, con
 cudaError_t launch_queries(const SceneView& s, const bf200_ray_v1* rays, uint64_t n, bf200_hit_v1* hits,
                            uint32_t* occluded, cudaStream_t stream) {
     if (hits != nullptr) {
-        cudaError_t e = s.sphere_count != 0U ? launch_pool<false>(k_query_closest<true>, n, stream, s, rays, n, hits)
-                                             : launch_pool<false>(k_query_closest<false>, n, stream, s, rays, n, hits);
+        cudaError_t e = s.sphere_count != 0U ? launch_pool<false>(k_query_closest<true>, n, stream, false, s, rays, n, hits)
+                                             : launch_pool<false>(k_query_closest<false>, n, stream, false, s, rays, n, hits);
         if (e == cudaSuccess) {
             const uint32_t blocks = static_cast<uint32_t>(std::min<uint64_t>((n + 127U) / 128U, 65535U));
             if (s.sphere_count != 0U) {
@@ -2582,8 +2581,8 @@ cudaError_t launch_queries(const SceneView& s, const bf200_ray_v1* rays, uint64_
         }
         return e;
     }
-    return s.sphere_count != 0U ? launch_pool<true>(k_query_occlusion<true>, n, stream, s, rays, n, occluded)
-                                : launch_pool<true>(k_query_occlusion<false>, n, stream, s, rays, n, occluded);
+    return s.sphere_count != 0U ? launch_pool<true>(k_query_occlusion<true>, n, stream, false, s, rays, n, occluded)
+                                : launch_pool<true>(k_query_occlusion<false>, n, stream, false, s, rays, n, occluded);
 }
 
 #endif  // BF200_KERNELS_MAIN_TU

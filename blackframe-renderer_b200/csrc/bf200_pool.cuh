@@ -419,6 +419,7 @@ __device__ __forceinline__ void pool_walk(const SceneView& s, Job& job, uint32_t
 // cache (no_instruction 3.2 stalls per issue).
 template <bool SPH>
 __global__ void __launch_bounds__(256) k_hits(SceneView s, Wavefront w) {
+    chain_begin();
     const uint32_t count = static_cast<uint32_t>(w.counters[kCounterTraced]);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
         const uint32_t slot = w.trace_queue[i];
@@ -497,6 +498,7 @@ struct TraceJob {
 template <bool SPH>
 __global__ void __launch_bounds__(kPoolThreads, kPoolBlocks) k_trace(SceneView s, Wavefront w) {
     extern __shared__ uint32_t pool[];
+    chain_begin();
     const uint32_t count = static_cast<uint32_t>(w.counters[kCounterTraced]);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         w.counters[3] += count;  // extension segments
@@ -582,6 +584,7 @@ struct OccludeJob {
 template <bool ADJ, bool SPH>
 __global__ void __launch_bounds__(kPoolThreads, kPoolBlocks) k_occlude(SceneView s, Wavefront w, AdjointView a) {
     extern __shared__ uint32_t pool[];
+    chain_begin();
     __shared__ double adjoint_sum[ADJ ? kAdjointWords : 1];
     if constexpr (ADJ) {
         adjoint_zero(adjoint_sum);
@@ -698,6 +701,7 @@ template <bool SPH>
 __global__ void __launch_bounds__(kPoolThreads, kPoolBlocks) k_query_closest(SceneView s, const bf200_ray_v1* rays,
                                                                              uint64_t n, bf200_hit_v1* hits) {
     extern __shared__ uint32_t pool[];
+    chain_begin();
     ClosestQuery job(rays, n, hits);
     pool_walk<false, SPH>(s, job, pool);
 }
@@ -706,6 +710,7 @@ template <bool SPH>
 __global__ void __launch_bounds__(kPoolThreads, kPoolBlocks) k_query_occlusion(SceneView s, const bf200_ray_v1* rays,
                                                                                uint64_t n, uint32_t* out) {
     extern __shared__ uint32_t pool[];
+    chain_begin();
     OcclusionQuery job(rays, n, out);
     pool_walk<true, SPH>(s, job, pool);
 }
@@ -713,7 +718,7 @@ __global__ void __launch_bounds__(kPoolThreads, kPoolBlocks) k_query_occlusion(S
 // Launches a pool kernel over `rays` rays at most: one resident wave of blocks, or as many as give
 // every lane a ray.
 template <bool ANY, class... Params, class... Args>
-cudaError_t launch_pool(void (*kernel)(Params...), uint64_t rays, cudaStream_t stream, Args... args) {
+cudaError_t launch_pool(void (*kernel)(Params...), uint64_t rays, cudaStream_t stream, bool chained, Args... args) {
     int device = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&device);
     if (e == cudaSuccess) {
@@ -729,8 +734,8 @@ cudaError_t launch_pool(void (*kernel)(Params...), uint64_t rays, cudaStream_t s
     const uint64_t wave = static_cast<uint64_t>(sms) * kPoolBlocks;
     const uint64_t need = (rays + kPoolThreads - 1U) / kPoolThreads;
     const uint32_t blocks = static_cast<uint32_t>(need < wave ? (need == 0U ? 1U : need) : wave);
-    kernel<<<blocks, kPoolThreads, kPoolSharedBytes<ANY>, stream>>>(args...);
-    return cudaGetLastError();
+    return launch_chained(kernel, blocks, static_cast<uint32_t>(kPoolThreads), kPoolSharedBytes<ANY>, stream, chained,
+                          args...);
 }
 
 }  // namespace bf200
