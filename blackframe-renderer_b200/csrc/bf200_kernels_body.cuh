@@ -353,6 +353,32 @@ __device__ __forceinline__ int triangle_test(float4 v0, float4 v1, float4 v2, F3
     return kTriHit;
 }
 
+// Whether two edge functions certainly have opposite signs by single precision, so that the ray misses
+// the triangle (what triangle_test, in double, finds first). Vertex and edge differences, products and
+// sums round at most seven times along any term of e = d . (p x f), and the terms sum to at most
+// 2 |d|_1 |p|_max |f|_max, so the error is below 14.1 u |d|_1 |p|_max |f|_max; 20u is asked for. Values in
+// the reach of subnormal products decide nothing, nor does anything that can overflow: 4 |p|_max |f|_max
+// and its product with |d|_1 bound every intermediate and are infinite first.
+__device__ __forceinline__ bool certain_miss(float4 v0, float4 v1, float4 v2, F3 o, F3 d, float d_sum) {
+    const F3 p0{v0.x - o.x, v0.y - o.y, v0.z - o.z}, p1{v1.x - o.x, v1.y - o.y, v1.z - o.z},
+        p2{v2.x - o.x, v2.y - o.y, v2.z - o.z};
+    const F3 f0{v2.x - v1.x, v2.y - v1.y, v2.z - v1.z}, f1{v0.x - v2.x, v0.y - v2.y, v0.z - v2.z},
+        f2{v1.x - v0.x, v1.y - v0.y, v1.z - v0.z};
+    const auto largest = [](F3 a, F3 b, F3 c) {
+        return fmaxf(fmaxf(fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(a.z), fabsf(b.x))),
+                           fmaxf(fmaxf(fabsf(b.y), fabsf(b.z)), fmaxf(fabsf(c.x), fabsf(c.y)))),
+                     fabsf(c.z));
+    };
+    const auto edge = [&](F3 p, F3 f) {
+        const F3 c{fmaf(p.y, f.z, -(p.z * f.y)), fmaf(p.z, f.x, -(p.x * f.z)), fmaf(p.x, f.y, -(p.y * f.x))};
+        return fmaf(d.x, c.x, fmaf(d.y, c.y, d.z * c.z));
+    };
+    const float bound = fmaxf(4.0F * largest(p0, p1, p2) * largest(f0, f1, f2) * d_sum * (5.0F * 5.9604645e-8F),
+                              1e-30F * (1.0F + d_sum));
+    const float e0 = edge(p1, f0), e1 = edge(p2, f1), e2 = edge(p0, f2);
+    return (e0 > bound || e1 > bound || e2 > bound) && (e0 < -bound || e1 < -bound || e2 < -bound);
+}
+
 // ------------------------------------------------------------------------------------------------
 // BVH traversal
 // ------------------------------------------------------------------------------------------------

@@ -296,16 +296,28 @@ __device__ __forceinline__ void pool_walk(const SceneView& s, Job& job, uint32_t
                 const uint32_t first = packed >> kLeafCountBits;
                 const uint32_t n = SPH && op == kPoolSphere ? 1U : (packed & (kMaxLeafSize - 1)) + 1U;
                 const float4* record = s.leaf_tris + 3ULL * first;
-                float4 r0 = record[0], r1 = record[1], r2 = record[2];
-                for (uint32_t j = 0; j < n; ++j) {
-                    const uint32_t leaf = first + j;
-                    const float4 v0 = r0, v1 = r1, v2 = r2;
-                    if (j + 1U < n) {  // the next triangle loads while this one is tested
-                        record += 3;
-                        r0 = record[0];
-                        r1 = record[1];
-                        r2 = record[2];
+                // most triangles of a leaf are certain misses; the double test then runs for the rest,
+                // one per round, instead of for every triangle with whichever lanes still need it (trace and
+                // k_hits, BVH stress 16 spp: 79.4 ms and 74.4 ms with the filter; Cornell box with spheres,
+                // 256 spp: 29.3 and 27.1)
+                uint32_t candidates = 1U;
+                if constexpr (!ANY) {
+                    if (!SPH || op == kPoolLeaf) {
+                        const float d_sum = fabsf(d.x) + fabsf(d.y) + fabsf(d.z);
+                        candidates = 0U;
+                        for (uint32_t j = 0; j < n; ++j) {
+                            candidates |= certain_miss(record[3U * j], record[3U * j + 1U], record[3U * j + 2U], o, d,
+                                                       d_sum)
+                                              ? 0U
+                                              : 1U << j;
+                        }
                     }
+                }
+                while (candidates != 0U) {
+                    const uint32_t j = static_cast<uint32_t>(__ffs(static_cast<int>(candidates))) - 1U;
+                    candidates &= candidates - 1U;
+                    const uint32_t leaf = first + j;
+                    const float4 v0 = record[3U * j], v1 = record[3U * j + 1U], v2 = record[3U * j + 2U];
                     int res = kTriMiss;
                     float t = 0.0F;
                     if (SPH && op == kPoolSphere) {
