@@ -54,14 +54,14 @@ FILM_SAMPLE_BYTES = 24
 # segment for occlude): trace reads the ray (28) and writes the hit (20); shade owns the rest of the
 # extension segment's 240 B; occlude the whole shadow segment
 STAGE_BYTES_PER_UNIT = {"trace": 48, "shade": EXTENSION_SEGMENT_BYTES - 48, "occlude": SHADOW_SEGMENT_BYTES}
-STAGE_KERNELS = {"trace": "k_trace", "shade": "k_shade<kind> x4 + route/shadow compaction",
+STAGE_KERNELS = {"trace": "k_trace + k_hits", "shade": "k_shade<kind> x4 + route/shadow compaction",
                  "occlude": "k_occlude"}
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per processed unit, per workload, from
 # one ncu capture of a full-wavefront launch of each stage's kernels in this build (the stage
 # kernels' launches at 2,097,152 slots)
 MEASURED_TRAFFIC_PER_UNIT = {
-    "cornell_spheres_256": {"trace": 56.5, "shade": 372.0, "occlude": None},
-    "bvh_stress_1080p": {"trace": 203.0, "shade": None, "occlude": None},
+    "cornell_spheres_256": {"trace": None, "shade": None, "occlude": None},
+    "bvh_stress_1080p": {"trace": 308.0, "shade": None, "occlude": None},
 }
 
 
@@ -514,8 +514,7 @@ def run_adjoint(args, torch, rank):
         torch.cuda.synchronize()
         e2e_ms.append((time.perf_counter() - t0) * 1000.0)
     e2e_value = paths * len(e2e_ms) / (sum(e2e_ms) / 1000.0)
-    # one more call, untimed, with the host-driven loop: profilers see the replay kernels of this
-    # call (the device-side loop graph of the timed calls hides its kernels from them)
+    # one more call, untimed, that waits for every iteration, for profilers to find its launches in order
     options.instrumentation = 1
     adjoint()
     options.instrumentation = 0
