@@ -1245,20 +1245,11 @@ __device__ __forceinline__ float scale_radiometric(float value, const float (&nu
     if (value == 0.0F) {
         return 0.0F;
     }
-    {
-        float direct = value, least = value;
-        for (int i = 0; i < n; ++i) {
-            direct *= num[i];
-            least = fminf(least, fminf(num[i], direct));
-        }
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            direct /= den[i];
-            least = fminf(least, fminf(den[i], direct));
-        }
-        if (least >= kMinNormal && direct <= kMaxFloat) {
-            return direct;
-        }
+    // factors beyond the n-th are 1, which changes no product
+    const float all[4] = {value, num[0], n > 1 ? num[1] : 1.0F, n > 2 ? num[2] : 1.0F};
+    float direct;
+    if (Factors<4, 3>(all, den).direct(direct)) {
+        return direct;
     }
     return split_radiometric(value, n, Factors<3, 3>({num[0], num[1], num[2]}, den), lane);
 }

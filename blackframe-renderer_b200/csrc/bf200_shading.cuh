@@ -370,10 +370,11 @@ BF_BLOCK void unit_segment(F3 origin, F3 endpoint, F3 expected, F3& direction,
 
 // The reference multiplies and divides frexp significands and restores the exponent at the end, so that
 // no partial result can leave the float range. Rounding does not depend on the exponent: while every
-// factor and every partial result is a normal number, the plain products and quotients have the same
-// bits. That is nearly always so, and several times shorter (about 20 instructions for a light's
-// seven factors over two, against 250); everything else -- zeros, subnormals, overflow, invalid
-// factors -- takes the exponent-split form. Cornell box with spheres, 256 spp: shading
+// factor and every partial result is a normal number greater than the smallest one, the plain products and
+// quotients have the same bits (a result below the normal range may round up to its smallest number, and
+// only the split form then keeps all 24 bits for the next step). That is nearly always so, and several
+// times shorter (about 20 instructions for a light's seven factors over two, against 250); everything else
+// -- zeros, subnormals, overflow, invalid factors -- takes the exponent-split form. Cornell box with spheres, 256 spp: shading
 // 44.8 -> 35.7 ms; BVH-stress frame, 16 samples: 45.3 -> 39.9 ms.
 constexpr float kMinNormal = 1.17549435e-38F, kMaxFloat = 3.40282347e+38F;
 
@@ -391,7 +392,7 @@ struct Factors {
             den[i] = d[i];
         }
     }
-    // num[0] * num[1] * ... / den[0] / ..., true when every step of it is normal
+    // num[0] * num[1] * ... / den[0] / ..., true when every step of it is above the smallest normal number
     __device__ __forceinline__ bool direct(float& result) const {
         float product = num[0], least = num[0];
 #pragma unroll
@@ -405,7 +406,7 @@ struct Factors {
             least = fminf(least, fminf(den[i], product));
         }
         result = product;
-        return least >= kMinNormal && product <= kMaxFloat;
+        return least > kMinNormal && product <= kMaxFloat;
     }
 };
 
@@ -525,7 +526,7 @@ __device__ __forceinline__ float positive_product2(float a, float b, Lane& lane)
     if (b == 0.0F) {
         return 0.0F;
     }
-    const float direct = a * b;
+    const float direct = a * b;  // one rounding: 2^-126 itself is what the split form's two give too
     if (fminf(fminf(a, b), direct) >= kMinNormal && direct <= kMaxFloat) {
         return direct;
     }

@@ -1,6 +1,7 @@
-"""The rule by which shading multiplies factors directly instead of by frexp significands
+"""The mathematics of the rule by which shading multiplies factors directly instead of by frexp significands
 (Factors::direct in bf200_shading.cuh): whenever it applies, both forms have the same bits. Restated
-here in numpy float32, whose operations round like the device's."""
+here in numpy float32, whose operations round like the device's; test_device_rules.py checks the
+header's own code."""
 import numpy as np
 import pytest
 
@@ -16,7 +17,7 @@ def direct(num, den):
     for v in den:
         product = product / v
         least = np.fmin(least, np.fmin(v, product))
-    return product, (least >= MIN_NORMAL) & (product <= MAX_FLOAT)
+    return product, (least > MIN_NORMAL) & (product <= MAX_FLOAT)
 
 
 def split(num, den, renormalise):
