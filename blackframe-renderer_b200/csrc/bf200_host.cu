@@ -1507,6 +1507,7 @@ BF200_EXPORT blackframe_status bf200_context_destroy(bf200_context* c) noexcept 
     }
     for (cudaStream_t st : c->shade_branches.stream) {
         if (st != nullptr) {
+            cudaStreamSynchronize(st);
             cudaStreamDestroy(st);
         }
     }

@@ -5,6 +5,7 @@
 
 #include <vector>
 
+#include "bf200_branches.h"
 #include "bf200_device.cuh"
 
 namespace bf200 {
@@ -47,11 +48,6 @@ cudaError_t launch_world_normals(const SceneView& s, uint32_t total, float4* out
 // shading and occlusion stages run as the path-replay adjoint's replay.
 // With `branches`, the Lambert kernel and the other shading kernels each go on a stream of their own,
 // forked and joined by the branches' events. `chained`: see launch_chained.
-constexpr uint32_t kShadeBranches = 3U;
-struct ShadeBranches {
-    cudaStream_t stream[kShadeBranches];
-    cudaEvent_t fork, join[kShadeBranches];
-};
 cudaError_t launch_stage(int stage, const SceneView& s, const Wavefront& w, const PathSource& src,
                          const TransportParams& p, uint32_t grid, cudaStream_t stream, uint32_t* launches,
                          const AdjointView* adjoint = nullptr, const ShadeBranches* branches = nullptr,

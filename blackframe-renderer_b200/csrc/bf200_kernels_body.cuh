@@ -2436,24 +2436,11 @@ BF200_SHADE_LAUNCHERS(true, false, false)
 template <bool ADJ, bool CONE, bool TREE>
 cudaError_t launch_shading(const SceneView& s, const Wavefront& w, const PathSource& src, const TransportParams& p,
                            uint32_t grid, const AdjointView& a, cudaStream_t stream, const ShadeBranches* branches) {
-    cudaStream_t on[kShadeBranches] = {stream, stream, stream};
-    cudaError_t e = branches != nullptr ? cudaEventRecord(branches->fork, stream) : cudaSuccess;
-    for (uint32_t k = 0; k < kShadeBranches && branches != nullptr && e == cudaSuccess; ++k) {
-        on[k] = branches->stream[k];
-        e = cudaStreamWaitEvent(on[k], branches->fork, 0);
-    }
-    if (e == cudaSuccess) {
+    return fork_join(branches, stream, [&](const cudaStream_t(&on)[kShadeBranches]) {
         launch_shade_lambert<ADJ, CONE, TREE>(s, w, src, p, grid, a, stream);
         launch_shade_others<ADJ, CONE, TREE>(s, w, src, p, grid, a, on);
-        e = cudaGetLastError();
-    }
-    for (uint32_t k = 0; k < kShadeBranches && branches != nullptr && e == cudaSuccess; ++k) {
-        e = cudaEventRecord(branches->join[k], on[k]);
-        if (e == cudaSuccess) {
-            e = cudaStreamWaitEvent(stream, branches->join[k], 0);
-        }
-    }
-    return e;
+        return cudaGetLastError();
+    });
 }
 
 // ------------------------------------------------------------------------------------------------
