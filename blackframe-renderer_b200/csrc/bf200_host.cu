@@ -3410,6 +3410,10 @@ BF200_EXPORT blackframe_status bf200_render_films_device(bf200_context* c, const
     return run_batch(c, jobs + measured, job_count - measured, std::min<uint32_t>(best, job_count - measured));
 }
 
+// The most staging that a context keeps for ray queries (1.6 million closest-hit rays). A larger call's
+// copies take longer than an allocation, so it allocates its own memory and releases it.
+constexpr size_t kKeptQueryBytes = size_t(128) << 20;
+
 static blackframe_status run_queries(bf200_context* c, const bf200_scene* s, const bf200_ray_v1* rays, uint64_t n,
                                      bf200_hit_v1* hits, uint32_t* occluded) {
     if (c == nullptr || s == nullptr || (n != 0 && rays == nullptr)) {
@@ -3423,13 +3427,19 @@ static blackframe_status run_queries(bf200_context* c, const bf200_scene* s, con
     // a release of each per call, 20,001 rays took 1.0 ms, and 0.29 ms without
     const size_t out_bytes = n * (hits != nullptr ? sizeof(bf200_hit_v1) : sizeof(uint32_t));
     const size_t ray_bytes = (n * sizeof(bf200_ray_v1) + 255) & ~size_t(255);
-    if (const auto st = grow_workspace(c, &c->batch_staging, &c->batch_staging_bytes, ray_bytes + out_bytes,
-                                       "query staging");
-        st != BLACKFRAME_STATUS_SUCCESS) {
-        return st;
+    const size_t need = ray_bytes + out_bytes;
+    void* released = nullptr;  // a large call's own memory
+    if (need <= std::max(kKeptQueryBytes, c->batch_staging_bytes)) {
+        if (const auto st = grow_workspace(c, &c->batch_staging, &c->batch_staging_bytes, need, "query staging");
+            st != BLACKFRAME_STATUS_SUCCESS) {
+            return st;
+        }
+    } else if (const cudaError_t m = cudaMalloc(&released, need); m != cudaSuccess) {
+        return cuda_fail(c, m, "query staging");
     }
-    auto* d_rays = static_cast<bf200_ray_v1*>(c->batch_staging);
-    void* d_out = static_cast<char*>(c->batch_staging) + ray_bytes;
+    char* const staging = static_cast<char*>(released != nullptr ? released : c->batch_staging);
+    auto* d_rays = reinterpret_cast<bf200_ray_v1*>(staging);
+    void* d_out = staging + ray_bytes;
     cudaError_t e = cudaMemcpyAsync(d_rays, rays, n * sizeof(bf200_ray_v1), cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess) {
         e = launch_queries(s->view, d_rays, n, hits != nullptr ? static_cast<bf200_hit_v1*>(d_out) : nullptr,
@@ -3441,6 +3451,9 @@ static blackframe_status run_queries(bf200_context* c, const bf200_scene* s, con
     }
     const cudaError_t done = cudaStreamSynchronize(c->stream);
     e = e == cudaSuccess ? done : e;
+    if (released != nullptr) {
+        cudaFree(released);
+    }
     return e == cudaSuccess ? BLACKFRAME_STATUS_SUCCESS : cuda_fail(c, e, "query");
 }
 

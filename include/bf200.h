@@ -472,7 +472,7 @@ BF200_EXTERN_C BF200_EXPORT blackframe_status bf200_context_create(int32_t devic
 BF200_EXTERN_C BF200_EXPORT blackframe_status bf200_context_destroy(bf200_context* context)
     BF200_NOEXCEPT;
 /* Device memory the context holds: its wavefront arena and the grow-only workspaces of the film,
- * batch, cone and adjoint calls, in bytes (not its scenes). Replaces
+ * batch, cone, adjoint and ray-query calls (queries keep 128 MiB at most), in bytes (not its scenes). Replaces
  * CudaWavefrontTransportWorkspace::device_size_bytes (WavefrontTransport.hpp:166). */
 BF200_EXTERN_C BF200_EXPORT blackframe_status bf200_context_device_bytes(const bf200_context* context,
                                                                           uint64_t* out_bytes) BF200_NOEXCEPT;
