@@ -183,9 +183,9 @@ class CpuReference:
     is loaded on this path."""
 
     def __init__(self, workload):
-        from oracle.bindings import CheckerError, Oracle, Reference, reference_available
-        if not reference_available():
-            raise CheckerError("the CPU reference arm needs oracle/_ref/libbfref.so (oracle/Makefile, target ref)")
+        from oracle.bindings import CheckerError, Oracle, Reference
+        if reference_absent():
+            raise CheckerError(reference_absent())
         self.workload = workload
         self.builder, self.options, (self.width, self.height, self.spp) = scenes.build_workload(workload)
         self.kind = "port" if workload in PORT_BASELINE_WORKLOADS else "reference"
@@ -229,6 +229,21 @@ class CpuReference:
                 "oracle/_ref: the reference's trace_scene_mis with its analytic accel")
         return (f"{n} random (pixel, sample) paths of {self.workload} per step, primary rays of the reference's "
                 f"PinholeCamera, traced by {what} on {self.threads} threads")
+
+
+def reference_absent():
+    """Why the CPU reference cannot run here (one line), or None."""
+    from oracle.bindings import reference_available
+    return None if reference_available() else ("the CPU reference arm needs oracle/_ref/libbfref.so (oracle/Makefile, "
+                                               "target ref, from the reference sources)")
+
+
+def cpu_baseline(workload, target_seconds):
+    """The JSON line's record of the CPU reference's rate; a machine without the reference build says so."""
+    if reference_absent():
+        return {"unavailable": reference_absent()}
+    rate, threads, kind, sample, _, _ = cpu_sample_rate(workload, target_seconds=target_seconds)
+    return {"value": rate, "unit": "path samples/s", "cores": threads, "kind": kind, "sample": sample}
 
 
 def cpu_sample_rate(workload, target_seconds=15.0):
@@ -768,6 +783,9 @@ def run_reference_arm(args, rank, world):
     warm-up step traces one path per thread)."""
     if rank != 0:
         return
+    if reference_absent():
+        print(json.dumps({"impl": "reference", "unavailable": reference_absent()}), flush=True)
+        return
     ref = CpuReference(args.workload)
     for _ in range(args.warmup):
         ref.run(ref.threads)
@@ -802,7 +820,12 @@ def run_reference_cuda_arm(args, rank, world):
     if rank != 0:
         return
     import torch
-    from oracle.bindings import ReferenceCuda
+    from oracle.bindings import ReferenceCuda, reference_cuda_available
+    if reference_absent() or not reference_cuda_available():  # the CPU build makes its camera rays
+        print(json.dumps({"impl": "reference-cuda", "unavailable":
+                          "the reference CUDA arm needs oracle/_ref/libbfref.so and libbfrefcuda.so (oracle/Makefile, "
+                          "targets ref and refcuda, from the reference sources)"}), flush=True)
+        return
     builder, options, (width, height, spp) = scenes.build_workload(args.workload)
     ref = ReferenceCuda()
     t0 = time.perf_counter()
@@ -1113,9 +1136,7 @@ def main():
     scene.close()
     ctx.close()
     if rank == 0 and not args.no_cpu_baseline and args.workload in scenes.WORKLOADS:
-        rate, threads, kind, sample, _, _ = cpu_sample_rate(args.workload, target_seconds=args.reference_seconds)
-        line["cpu_baseline"] = {"value": rate, "unit": "path samples/s", "cores": threads, "kind": kind,
-                                "sample": sample}
+        line["cpu_baseline"] = cpu_baseline(args.workload, args.reference_seconds)
     if distributed:
         dist.barrier()
         dist.destroy_process_group()
