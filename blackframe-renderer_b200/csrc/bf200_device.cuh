@@ -32,11 +32,15 @@ struct alignas(128) BvhNode4 {
 };
 
 constexpr int kLeafCountBits = 3;
+// Triangles of a leaf, in both BLAS builds (leaf codes could count more; the walk's shared arrays could not).
+constexpr int kMaxLeafTriangles = 4;
 // Scenes with at most this many instances test every instance box up front; larger ones walk a
 // TLAS over the instances' world boxes.
 constexpr uint32_t kEagerInstances = 32;
 constexpr int kMaxLeafSize = 1 << kLeafCountBits;
-constexpr int kTraversalStack = 128;  // up to 32 instance entries plus one BLAS walk
+// Stack entries of a walk: up to 32 instance entries or a TLAS walk, plus one BLAS walk. Scene creation
+// refuses deeper trees; the walks do not check.
+constexpr int kTraversalStack = 128;
 
 struct LightInfo {
     uint32_t instance;

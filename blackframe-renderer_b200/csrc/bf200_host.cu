@@ -223,8 +223,7 @@ struct Prim {
     uint32_t index;
 };
 
-constexpr int kLeafSize = 4;
-static_assert(kLeafSize < static_cast<int>(kSphereLeafCount) && kSphereLeafCount == kMaxLeafSize,
+static_assert(kMaxLeafTriangles < static_cast<int>(kSphereLeafCount) && kSphereLeafCount == kMaxLeafSize,
               "triangle leaves never carry the sphere leaf count");
 constexpr int kBins = 16;
 
@@ -241,7 +240,7 @@ struct Builder {
     const float* positions;  // geometry-local base
     const uint32_t* tris;
     uint32_t max_depth = 0;
-    int leaf_limit = kLeafSize;
+    int leaf_limit = kMaxLeafTriangles;
     bool instance_leaves = false;  // TLAS: one instance per leaf, encoded as ~instance
     int parallel_levels = 0;       // levels whose large right subtrees go to their own thread
 
@@ -457,7 +456,7 @@ uint32_t build_blas(const bf200_scene_desc_v1& d, uint32_t g, std::vector<BvhNod
         ++b.parallel_levels;  // up to 2^levels subtrees in flight, at most 32
     }
     const uint32_t root = static_cast<uint32_t>(nodes.size());
-    if (static_cast<int>(prims.size()) <= kLeafSize) {
+    if (static_cast<int>(prims.size()) <= kMaxLeafTriangles) {
         nodes.push_back(BvhNode{});
         const Box lb = b.bounds(0, static_cast<int>(prims.size()));
         const int leaf = b.make_leaf(0, static_cast<int>(prims.size()));

@@ -35,7 +35,6 @@
 namespace bf200 {
 namespace {
 
-constexpr int kLbvhLeaf = 4;  // the host build's leaf bound (kLeafSize)
 constexpr uint32_t kLbvhThreads = 256;
 constexpr int kMortonBits = 63;
 
@@ -191,7 +190,7 @@ __global__ void __launch_bounds__(kLbvhThreads) k_lbvh_hierarchy(const unsigned 
     const int split = i + s * d + min(d, 0);
     const int first = min(i, j), last = max(i, j);
     const int left_count = split - first + 1, right_count = last - split;
-    const bool left_leaf = left_count <= kLbvhLeaf, right_leaf = right_count <= kLbvhLeaf;
+    const bool left_leaf = left_count <= kMaxLeafTriangles, right_leaf = right_count <= kMaxLeafTriangles;
     const int left = left_leaf ? leaf_code(leaf_base + static_cast<uint32_t>(first), left_count)
                                : static_cast<int>(node_base) + split;
     const int right = right_leaf ? leaf_code(leaf_base + static_cast<uint32_t>(split + 1), right_count)
@@ -208,7 +207,7 @@ __global__ void __launch_bounds__(kLbvhThreads) k_lbvh_hierarchy(const unsigned 
         parent[split + 1] = i;
     }
     // w: the node is referenced (its range exceeds a leaf); the root always is
-    ranges[i] = make_int4(first, split, last, (last - first + 1 > kLbvhLeaf || i == 0) ? 1 : 0);
+    ranges[i] = make_int4(first, split, last, (last - first + 1 > kMaxLeafTriangles || i == 0) ? 1 : 0);
 }
 
 __global__ void __launch_bounds__(kLbvhThreads) k_lbvh_leaves(const float* __restrict__ positions,
@@ -269,7 +268,7 @@ __global__ void __launch_bounds__(kLbvhThreads) k_lbvh_boxes(BvhNode* __restrict
     for (int slot = 0; slot < 2; ++slot) {
         const int first = slot == 0 ? r.x : r.y + 1;
         const int last = slot == 0 ? r.y : r.z;
-        if (last - first + 1 > kLbvhLeaf) {
+        if (last - first + 1 > kMaxLeafTriangles) {
             continue;
         }
         float lo[3] = {inf, inf, inf}, hi[3] = {-inf, -inf, -inf};
@@ -306,7 +305,7 @@ uint32_t blocks(uint32_t n) {
 cudaError_t build_blas_lbvh(const float* positions, uint32_t vertex_count, const uint32_t* triangles, uint32_t n,
                             uint32_t node_base, uint32_t leaf_base, std::vector<BvhNode>& nodes,
                             std::vector<float4>& leaf_tris, cudaStream_t stream) {
-    if (n <= static_cast<uint32_t>(kLbvhLeaf)) {
+    if (n <= static_cast<uint32_t>(kMaxLeafTriangles)) {
         return cudaErrorInvalidValue;  // tiny geometries take the host build
     }
     const uint32_t tiles = (n + kCompactTile - 1) / kCompactTile;

@@ -45,9 +45,12 @@ enum PoolWord : int {
 constexpr int kPoolWords = kPoolFrames + kPoolStack;
 constexpr uint32_t kPoolSpMask = 0xFFU, kPoolAxes = 0x700U, kPoolFound = 0x800U, kPoolFailed = 0x1000U;
 constexpr int kPoolAxesShift = 8;
-// One operation's leaf triangles, per warp: the tests of all its lanes (at most 4 each), and the lane and
+static_assert(kTraversalStack <= static_cast<int>(kPoolSpMask), "a stack size fits its bits");
+// One operation's leaf triangles, per warp: the tests of all its lanes, and the lane and
 // ray that asked for each.
-constexpr uint32_t kPoolTests = 128U;
+constexpr uint32_t kPoolTests = 32U * kMaxLeafTriangles;
+static_assert(kMaxLeafTriangles < 8 && kPoolRays<true> <= 8,
+              "leaf sizes are dealt by three ballots, and a test's lane and ray fit one byte");
 template <bool ANY>
 constexpr int kPoolRayWords = kPoolWords * kPoolRays<ANY> * kPoolThreads;
 template <bool ANY>
