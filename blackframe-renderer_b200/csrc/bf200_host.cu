@@ -58,6 +58,7 @@ struct bf200_context {
     void* batch_staging = nullptr;  // device copies of host path inputs and results, and of query rays and answers
     size_t batch_staging_bytes = 0;
     bf200::ShadeBranches shade_branches{};
+    cudaEvent_t iteration_events[2] = {};  // blocking waits of the streamed loop (IterationWait)
     // film batches (bf200_render_films_device): one stream, event, arena slice, pinned counter
     // block and radiance buffer per lane, kept across calls
     std::vector<cudaStream_t> lane_streams;
@@ -1156,6 +1157,55 @@ void wavefront_report(const bf200_context* c, const bf200_scene* s, const PathSo
     report->iterations += iterations;
 }
 
+// The streamed loop's wait for an iteration's outcome, in the way the device's scheduling flags ask for. A device
+// set to blocking waits (cudaDeviceScheduleBlockingSync) blocks on an event behind the iteration; otherwise
+// the outcome is polled in pinned memory, and the processor is offered to other threads between polls unless
+// the device is set to spin.
+struct IterationWait {
+    cudaStream_t stream = nullptr;
+    cudaEvent_t* events = nullptr;  // two, for the iterations in flight; null: poll
+    bool yields = true;
+
+    cudaError_t begin(bf200_context* c) {
+        stream = c->stream;
+        unsigned int flags = 0;
+        cudaError_t e = cudaGetDeviceFlags(&flags);
+        yields = (flags & cudaDeviceScheduleMask) != cudaDeviceScheduleSpin;
+        if (e != cudaSuccess || (flags & cudaDeviceScheduleMask) != cudaDeviceScheduleBlockingSync) {
+            return e;
+        }
+        events = c->iteration_events;
+        for (int k = 0; k < 2 && e == cudaSuccess; ++k) {
+            if (events[k] == nullptr) {
+                e = cudaEventCreateWithFlags(&events[k], cudaEventDisableTiming | cudaEventBlockingSync);
+            }
+        }
+        return e;
+    }
+    // after the launches of iteration `index`
+    cudaError_t queued(uint64_t index) const {
+        return events != nullptr ? cudaEventRecord(events[index % 2U], stream) : cudaSuccess;
+    }
+    // until iteration `index`, the one before the last queued, has written its outcome
+    cudaError_t wait(uint64_t index, const volatile unsigned long long* outcome) const {
+        if (events != nullptr) {
+            return cudaEventSynchronize(events[index % 2U]);
+        }
+        for (uint32_t polls = 1U; *outcome == 0ULL; ++polls) {
+            if (polls % 4096U == 0U) {  // a failed stream writes no outcome
+                const cudaError_t state = cudaStreamQuery(stream);
+                if (state != cudaErrorNotReady) {  // nothing left to run: the outcome has been written
+                    return state;
+                }
+            }
+            if (yields && polls % 64U == 0U) {
+                std::this_thread::yield();
+            }
+        }
+        return cudaSuccess;
+    }
+};
+
 // The persistent wavefront, its iterations queued by the host one ahead of the GPU: while iteration i + 1
 // runs, the host reads how iteration i ended from pinned memory, so the GPU does not wait for the host,
 // and one idle iteration is queued past the last. It stops at the same iteration bound as the
@@ -1187,6 +1237,10 @@ blackframe_status run_wavefront_streamed(bf200_context* c, const bf200_scene* s,
     if (const auto b = ensure_shade_branches(c); b != BLACKFRAME_STATUS_SUCCESS) {
         return b;
     }
+    IterationWait wait;
+    if ((e = wait.begin(c)) != cudaSuccess) {
+        return cuda_fail(c, e, "wavefront wait");
+    }
     uint32_t launches = 0;
     uint64_t queued = 0, ended = 0;
     bool drained = false;
@@ -1199,20 +1253,14 @@ blackframe_status run_wavefront_streamed(bf200_context* c, const bf200_scene* s,
             e = launch_iteration_end(w, src.total, outcomes + queued % kOutcomes, st, chained);
             ++launches;
         }
+        if (e == cudaSuccess) {
+            e = wait.queued(queued);
+        }
         if (++queued < 2U || e != cudaSuccess) {
             continue;
         }
         // the outcome of the iteration before the one just queued
-        for (uint32_t spins = 1U; outcomes[ended % kOutcomes] == 0ULL && e == cudaSuccess; ++spins) {
-            if (spins % 4096U != 0U) {
-                continue;
-            }
-            const cudaError_t state = cudaStreamQuery(st);
-            if (state == cudaSuccess) {  // nothing left to run: the outcome has been written
-                break;
-            }
-            e = state == cudaErrorNotReady ? cudaSuccess : state;
-        }
+        e = wait.wait(ended, outcomes + ended % kOutcomes);
         drained = e == cudaSuccess && outcomes[ended % kOutcomes] == kIterationDrained;
         ++ended;
     }
@@ -1511,7 +1559,7 @@ BF200_EXPORT blackframe_status bf200_context_destroy(bf200_context* c) noexcept 
         }
     }
     for (cudaEvent_t ev : {c->shade_branches.fork, c->shade_branches.join[0], c->shade_branches.join[1],
-                           c->shade_branches.join[2]}) {
+                           c->shade_branches.join[2], c->iteration_events[0], c->iteration_events[1]}) {
         if (ev != nullptr) {
             cudaEventDestroy(ev);
         }
