@@ -235,7 +235,8 @@ struct Wavefront {
     // counters: [0] shadow queue size, [1] next path to claim, [2] active slots,
     //           [3] extension segments, [4] shadow segments, [5] failed lanes,
     //           [6] first failure path (min), [7] first failure code, [8] k_trace fetch cursor,
-    //           [9] iterations (k_iteration_end), [11..14] the cone-carrying kernels' stage counts, [15] k_occlude fetch cursor, [16] traced slots
+    //           [11..14] the cone-carrying kernels' stage counts, [15] k_occlude fetch cursor,
+    //           [16] traced slots
     unsigned long long* counters;
 };
 

@@ -1683,7 +1683,7 @@ BF200_EXPORT blackframe_status bf200_scene_create(bf200_context* c, const bf200_
             scene->blas_roots.push_back(g.z);
         }
         const auto t_instances = Clock::now();
-        // instance ranges on the traversal stack carry 14-bit first indices
+        // the interface's limit, well inside the traversal stack's instance entries
         if (d->instance_count >= (1U << 14)) {
             return fail(c, BLACKFRAME_STATUS_OUT_OF_RANGE, "more than 16383 instances");
         }

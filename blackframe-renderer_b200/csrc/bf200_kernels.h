@@ -66,8 +66,8 @@ cudaError_t build_blas_lbvh(const float* positions, uint32_t vertex_count, const
                             uint32_t node_base, uint32_t leaf_base, std::vector<BvhNode>& nodes,
                             std::vector<float4>& leaf_tris, cudaStream_t stream);
 // Queues k_iteration_end, which ends one iteration of the loop that the host queues: it accumulates the
-// shadow segments (counters[4]), counts iterations (counters[9]), clears the per-iteration counters and
-// writes kIterationMore or kIterationDrained to *outcome, in pinned host memory.
+// shadow segments (counters[4]), clears the per-iteration counters and writes kIterationMore or
+// kIterationDrained to *outcome, in pinned host memory.
 constexpr unsigned long long kIterationMore = 1ULL, kIterationDrained = 2ULL;
 cudaError_t launch_iteration_end(const Wavefront& w, uint64_t total, volatile unsigned long long* outcome,
                                  cudaStream_t stream, bool chained);

@@ -513,15 +513,12 @@ __device__ __forceinline__ int hit_children(const RayInv& r, const BvhNode4& n, 
 // Stack entries of both traversals: a BLAS node index (>= 0), a BLAS leaf (the node's child code,
 // in [-2^30, 0): ~child = first_leaf_triangle << 3 | (count - 1)), or an instance-level entry
 // below -2^30, kInstanceEntry + code with code < 2^30: a TLAS node (code = kTlasFlag | node) or an
-// instance range (code = first << 15 | count: the instances [first, first + count), index order).
+// instance (code = its index).
 constexpr int kInstanceEntry = INT_MIN;
 constexpr int kLeafEntryMin = -(1 << 30);
-constexpr int kInstanceBits = 15;
 constexpr uint32_t kTlasFlag = 1U << 29;
 
-__device__ __forceinline__ int instance_range(uint32_t first, uint32_t count) {
-    return kInstanceEntry + static_cast<int>((first << kInstanceBits) | count);
-}
+__device__ __forceinline__ int instance_entry(uint32_t inst) { return kInstanceEntry + static_cast<int>(inst); }
 
 __device__ __forceinline__ int tlas_entry(int node) {
     return kInstanceEntry + static_cast<int>(kTlasFlag | static_cast<uint32_t>(node));
@@ -2447,14 +2444,12 @@ cudaError_t launch_shading(const SceneView& s, const Wavefront& w, const PathSou
 // k_iteration_end: the end of one wavefront iteration that the host queued ahead
 // ------------------------------------------------------------------------------------------------
 
-// One thread. Accumulates the iteration's shadow segments, counts the iteration, clears the
-// per-iteration counters for the next one and tells the host (pinned memory) whether every path has
-// been traced.
+// One thread. Accumulates the iteration's shadow segments, clears the per-iteration counters for the next
+// one and tells the host (pinned memory) whether every path has been traced.
 __global__ void k_iteration_end(Wavefront w, uint64_t total, volatile unsigned long long* outcome) {
     chain_begin();
     unsigned long long* c = w.counters;
     c[4] += c[0];
-    ++c[9];
     const bool drained = c[2] == 0ULL && c[1] >= total;
     c[0] = 0ULL;
     c[2] = 0ULL;

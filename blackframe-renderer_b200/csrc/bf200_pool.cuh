@@ -195,7 +195,7 @@ __device__ __forceinline__ void pool_walk(const SceneView& s, Job& job, uint32_t
                     for (int c = 3; c >= 0; --c) {
                         if (tlas) {
                             kids[c] = kids[c] >= 0 ? tlas_entry(kids[c])
-                                                   : instance_range(static_cast<uint32_t>(~kids[c]), 1U);
+                                                   : instance_entry(static_cast<uint32_t>(~kids[c]));
                         }
                         if (c > 0 && c < count) {
                             ray.push(sp, kids[c]);
@@ -221,12 +221,9 @@ __device__ __forceinline__ void pool_walk(const SceneView& s, Job& job, uint32_t
                     flags = (flags & ~kPoolAxes) | ray.frame(o, d);
                     in_world = true;
                 } else {
-                    // an instance range (code = first << 15 | count) yields its first instance unless
-                    // the ray's visibility mask excludes it or its world box is not met
-                    const uint32_t inst = code >> kInstanceBits, count = code & ((1U << kInstanceBits) - 1U);
-                    if (count > 1U) {
-                        ray.push(sp, instance_range(inst + 1U, count - 1U));
-                    }
+                    // an instance (code = its index) is entered unless the ray's visibility mask excludes
+                    // it or its world box is not met
+                    const uint32_t inst = code;
                     const float4 blo = s.inst_world_box[2ULL * inst], bhi = s.inst_world_box[2ULL * inst + 1];
                     float near;
                     const RayInv r = make_ray_inv(o, d);
@@ -403,7 +400,7 @@ __device__ __forceinline__ void pool_walk(const SceneView& s, Job& job, uint32_t
                         float near;
                         if ((mask & __float_as_uint(blo.w)) != 0U &&
                             slab(r, blo.x, bhi.x, blo.y, bhi.y, blo.z, bhi.z, t_min, t_max, near)) {
-                            ray.push(sp, instance_range(static_cast<uint32_t>(inst), 1U));
+                            ray.push(sp, instance_entry(static_cast<uint32_t>(inst)));
                         }
                     }
                     next = ray.pop(sp);
@@ -716,7 +713,6 @@ template <bool SPH>
 __global__ void __launch_bounds__(kPoolThreads, kPoolBlocks) k_query_closest(SceneView s, const bf200_ray_v1* rays,
                                                                              uint64_t n, bf200_hit_v1* hits) {
     extern __shared__ uint32_t pool[];
-    chain_begin();
     ClosestQuery job(rays, n, hits);
     pool_walk<false, SPH>(s, job, pool);
 }
@@ -725,7 +721,6 @@ template <bool SPH>
 __global__ void __launch_bounds__(kPoolThreads, kPoolBlocks) k_query_occlusion(SceneView s, const bf200_ray_v1* rays,
                                                                                uint64_t n, uint32_t* out) {
     extern __shared__ uint32_t pool[];
-    chain_begin();
     OcclusionQuery job(rays, n, out);
     pool_walk<true, SPH>(s, job, pool);
 }
