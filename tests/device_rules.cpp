@@ -1,4 +1,4 @@
-// The device rules that tests check on the CPU: the shading header compiled for the host, where float
+// The device rules that tests check on the CPU: the shading and triangle headers compiled for the host, where
 // arithmetic rounds as on the device (no contraction), behind a few array functions.
 #include <cuda_runtime.h>
 
@@ -22,11 +22,13 @@ To bits_as(From v) {
 }
 inline float __int_as_float(int v) { return bits_as<float>(v); }
 inline int __float_as_int(float v) { return bits_as<int>(v); }
+inline float __double2float_rn(double v) { return static_cast<float>(v); }
 inline uint32_t __float_as_uint(float v) { return bits_as<uint32_t>(v); }
 inline int __ffsll(long long v) { return __builtin_ffsll(v); }
 }  // namespace
 
 #include "bf200_shading.cuh"
+#include "bf200_triangle.cuh"
 
 using namespace bf200;
 
@@ -91,6 +93,26 @@ void rule_split_mis_ratio(uint32_t heuristic, const float* less, const float* mo
 void rule_next_float(const float* v, uint32_t up, uint64_t n, float* out) {
     for (uint64_t i = 0; i < n; ++i) {
         out[i] = next_float(v[i], up != 0U);
+    }
+}
+
+// certain_miss of rays against triangles, and the whole test: 0 miss, 1 hit, 2 failure, with (t, barycentrics)
+void rule_triangles(const float* vertices, const float* origin, const float* direction, uint64_t n, uint8_t* certain,
+                    uint8_t* code, float* out) {
+    for (uint64_t i = 0; i < n; ++i) {
+        const float* p = vertices + 9 * i;
+        const float4 v0 = make_float4(p[0], p[1], p[2], 0.0F), v1 = make_float4(p[3], p[4], p[5], 0.0F),
+                     v2 = make_float4(p[6], p[7], p[8], 0.0F);
+        const F3 o{origin[3 * i], origin[3 * i + 1], origin[3 * i + 2]};
+        const F3 d{direction[3 * i], direction[3 * i + 1], direction[3 * i + 2]};
+        const float d_sum = fabsf(d.x) + fabsf(d.y) + fabsf(d.z);
+        certain[i] = certain_miss(v0, v1, v2, o, d, d_sum) ? 1 : 0;
+        TriangleHit hit{};
+        code[i] = static_cast<uint8_t>(triangle_test(v0, v1, v2, o, d, 0.0F, kInf, true, hit));
+        out[4 * i] = hit.t;
+        out[4 * i + 1] = hit.b0;
+        out[4 * i + 2] = hit.b1;
+        out[4 * i + 3] = hit.b2;
     }
 }
 }

@@ -1,6 +1,7 @@
-"""The single-precision rule that drops a leaf's triangles before the double test (certain_miss in
-bf200_kernels_body.cuh), restated in numpy: whenever it applies, two exact edge functions have opposite
-signs, which the double test answers with a miss."""
+"""The mathematics of the single-precision rule that drops a leaf's triangles before the double test
+(certain_miss in bf200_triangle.cuh), restated in numpy: whenever it applies, two exact edge functions have
+opposite signs, which the double test answers with a miss. test_device_rules.py checks the header's own
+code."""
 from fractions import Fraction
 
 import numpy as np

@@ -1,13 +1,15 @@
-"""The shading header's own product, MIS and stepping rules, compiled for the host (tests/device_rules.cpp):
-float32 operations round there as on the device, so what holds here holds in the kernels."""
+"""The device headers' own product, MIS and stepping rules and their triangle test, compiled for the host
+(tests/device_rules.cpp): operations round there as on the device, so what holds here holds in the kernels."""
 import ctypes as C
 import os
 import shutil
 import subprocess
+from fractions import Fraction
 
 import numpy as np
 import pytest
 
+from test_certain_miss import exact_signs
 from test_factor_products import F, MAX_FLOAT, MIN_NORMAL, factors
 
 CUDA_INCLUDE = "/usr/local/cuda/include"
@@ -110,3 +112,77 @@ def test_next_float_is_nextafter(rules):
         rules.rule_next_float(pointer(v), up, C.c_uint64(len(v)), pointer(out))
         with np.errstate(all="ignore"):
             assert same_bits(out, np.nextafter(v, F(np.inf) if up else F(-np.inf)))
+
+
+def triangles_and_rays(size, distance, n, seed):
+    """Triangles of a size seen from a distance, half of the rays aimed near an edge."""
+    rng = np.random.default_rng(seed)
+    v = (rng.normal(size=(n, 3, 3)) * size).astype(F)
+    w = rng.dirichlet((1.0, 1.0, 1.0), n)
+    w[::2, 0] = rng.normal(size=len(w[::2])) * 10.0 ** rng.uniform(-9.0, 0.0, len(w[::2]))
+    target = (w[:, :, None] * v).sum(axis=1) / w.sum(axis=1, keepdims=True)
+    d = rng.normal(size=(n, 3))
+    d = (d / np.linalg.norm(d, axis=1, keepdims=True)).astype(F)
+    return v, (target - distance * d).astype(F), d
+
+
+def run_triangles(rules, v, o, d):
+    n = len(v)
+    certain, code, out = np.zeros(n, np.uint8), np.zeros(n, np.uint8), np.zeros((n, 4), F)
+    rules.rule_triangles(pointer(np.ascontiguousarray(v)), pointer(o), pointer(d), C.c_uint64(n), pointer(certain),
+                         pointer(code), pointer(out))
+    return certain != 0, code, out
+
+
+@pytest.mark.parametrize("distance", [1e-3, 1.0, 30.0, 1e4, 1e12, 1e20])
+@pytest.mark.parametrize("size", [1e-12, 1e-3, 1.0, 1e18, 1e20])
+def test_certain_misses_are_misses(rules, size, distance):
+    v, o, d = triangles_and_rays(size, distance, 3000, abs(int(np.log10(size) * 31 + np.log10(distance))))
+    certain, code, _ = run_triangles(rules, v, o, d)
+    assert (code[certain] == 0).all()
+    for k in np.nonzero(certain)[0]:
+        signs = exact_signs(list(v[k]), o[k], d[k])
+        assert 1 in signs and -1 in signs, k
+    if size / distance >= 1e-3 and 1e-10 < size < 1e10:  # near enough for the rule to decide anything
+        assert certain.any()
+
+
+def test_non_finite_rays_are_no_certain_misses(rules):
+    v, o, d = triangles_and_rays(1.0, 1.0, 600, 3)
+    for k, value in enumerate((np.nan, np.inf, -np.inf)):
+        o[k::6, k] = value
+        d[3 + k::6, k] = value
+    certain, _, _ = run_triangles(rules, v, o, d)
+    assert not certain.any()
+
+
+def nearest_float(q):
+    """The float32 nearest to a Fraction, ties to even."""
+    f = F(float(q))
+    best = min((F(np.nextafter(f, F(-np.inf))), f, F(np.nextafter(f, F(np.inf)))),
+               key=lambda c: (abs(Fraction(float(c)) - q), int(c.view(np.uint32)) & 1))
+    return best
+
+
+@pytest.mark.parametrize("distance", [1.0, 100.0, 1e4])
+@pytest.mark.parametrize("size", [1e-12, 1.0, 1e12])
+def test_hits_are_the_exact_quotients_rounded_once(rules, size, distance):
+    v, o, d = triangles_and_rays(size, distance * size, 400, int(distance) + 5)
+    _, code, out = run_triangles(rules, v, o, d)
+    assert (code != 2).all() and (code == 1).mean() > 0.3
+    for k in range(len(v)):
+        p = [[Fraction(float(v[k][j][a])) - Fraction(float(o[k][a])) for a in range(3)] for j in range(3)]
+        r = [Fraction(float(x)) for x in d[k]]
+
+        def det(a, b, c):
+            return (a[0] * (b[1] * c[2] - b[2] * c[1]) - a[1] * (b[0] * c[2] - b[2] * c[0])
+                    + a[2] * (b[0] * c[1] - b[1] * c[0]))
+
+        e = [det(p[1], p[2], r), det(p[2], p[0], r), det(p[0], p[1], r)]
+        total = sum(e)
+        inside = total != 0 and (all(x >= 0 for x in e) or all(x <= 0 for x in e))
+        t = det(p[0], p[1], p[2]) / total if inside else None
+        assert (code[k] == 1) == (inside and t >= 0), k
+        if code[k] == 1:
+            wanted = [nearest_float(t)] + [nearest_float(x / total) for x in e]
+            assert same_bits(out[k] + F(0.0), np.array(wanted, F) + F(0.0)), k  # a zero's sign is not compared
