@@ -57,11 +57,11 @@ STAGE_BYTES_PER_UNIT = {"trace": 48, "shade": EXTENSION_SEGMENT_BYTES - 48, "occ
 STAGE_KERNELS = {"trace": "k_trace + k_hits", "shade": "k_shade<kind> x4 + route/shadow compaction",
                  "occlude": "k_occlude"}
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per processed unit, per workload, from
-# one ncu capture of a full-wavefront launch of each stage's kernels in this build (the stage
-# kernels' launches at 2,097,152 slots)
+# one ncu capture of a full-wavefront launch of the stage's kernels (2,097,152 slots,
+# profiles/stage_kernels_ray_pools_bvh_stress.md); None where the present kernels have not been captured
 MEASURED_TRAFFIC_PER_UNIT = {
     "cornell_spheres_256": {"trace": None, "shade": None, "occlude": None},
-    "bvh_stress_1080p": {"trace": 308.0, "shade": None, "occlude": None},
+    "bvh_stress_1080p": {"trace": 305.0, "shade": None, "occlude": None},
 }
 
 

@@ -8,17 +8,15 @@
 // whichever of its rays is due for it. BVH-stress frame, 1920 x 1080 x 16: k_trace 158 -> 91 ms with
 // k_hits, k_occlude 66 -> 35 ms; Cornell box with spheres, 256 x 256 x 256: 55 -> 31 and 22 -> 13.5 ms.
 // What bounds it now is latency at 16 warps per SM: the fixed latency of a visit's instructions and
-// the L2 round trips of its node, with 15 of 32 lanes active per instruction.
+// the L2 round trips of its node, with 16 (closest hits) and 18 (shadow rays) of 32 lanes per instruction.
 #pragma once
 
 namespace bf200 {
 
-// Rays per lane, threads per block, resident blocks per SM (the registers a walk needs allow four).
-// Measured on the BVH-stress frame (16 samples; trace + occlude): 1 ray 174 ms (6 blocks), 2 rays 130
-// ms, 3 rays 126 ms; 5 and 6 blocks with 2 rays 154 and 188 ms, from spills and the smaller L1. Shadow
-// rays deal their leaves' triangles over the warp (2 rays suffice then: occlude 34.6 -> 32.7 ms, Cornell
-// box with spheres 13.4 -> 12.8 ms). Closest hits do not: 89.7 -> 87.1 ms there, but 30.8 -> 32.5 ms in
-// the box, whose leaves hold one or two triangles.
+// Rays per lane, threads per block, resident blocks per SM (the registers a walk needs allow four; more
+// blocks spill and leave less L1). BVH-stress frame, 16 samples, trace + occlude: 174 ms with 1 ray, 130
+// with 2, 126 with 3. Shadow rays deal their leaves' triangles over the warp, and 2 rays suffice then
+// (occlude 34.6 -> 32.7 ms).
 constexpr int kPoolThreads = 128, kPoolBlocks = 4;
 template <bool ANY>
 constexpr int kPoolRays = ANY ? 2 : 3;
